@@ -381,6 +381,95 @@ void hostnet_from_aos(const BncBionData& aos, HostNet* hn) {
     for (uint32_t k = 0; k < aos.num_synapses; k++) hostnet_add_synapse(*hn, aos.synapses[k]);
 }
 
+namespace {
+
+// Lays an unbranched network out for k_diffusion_path: every component a path of at most
+// 128 segments whose connections are all intracellular.  Returns the slots per lane, 0
+// when the network is not of that kind (the CTA-tile kernel runs it).
+//
+// A warp holds 32 x R slots and whole components, in device order.  R = 2 has the lowest
+// time per slot once the chip is full (0.36 ns against 0.53 for R = 4, whose state leaves
+// 3 warps per scheduler), so R = 4 takes only components over 64 segments; R = 1 halves a
+// warp's work where the chip is idle anyway (64 neurons x 32: 34 us against 44).
+uint32_t path_layout(uint32_t n, uint32_t T, uint32_t cluster, const std::vector<uint32_t>& tile_seg_beg,
+                     const std::vector<uint32_t>& tile_edge_beg, const std::vector<uint16_t>& e_a,
+                     const std::vector<uint16_t>& e_b, const std::vector<uint8_t>& e_intra,
+                     const std::vector<float>& e_area, const std::vector<float>& e_dist, std::vector<uint32_t>* pt_seg,
+                     std::vector<float>* pt_area, std::vector<float>* pt_dist) {
+    if (cluster != 1 || n >= (1u << 31) - 1u) return 0;
+    // the (at most two) connections of each segment, in connection order
+    std::vector<uint32_t> nb((size_t)n * 2, UINT32_MAX), ne((size_t)n * 2, UINT32_MAX);
+    std::vector<uint8_t> deg(n, 0);
+    for (uint32_t t = 0; t < T; t++)
+        for (uint32_t e = tile_edge_beg[t]; e < tile_edge_beg[t + 1]; e++) {
+            const uint32_t a = tile_seg_beg[t] + e_a[e], b = tile_seg_beg[t] + e_b[e];
+            if (a == b || !e_intra[e] || deg[a] == 2 || deg[b] == 2) return 0;
+            // a contact area or length outside these (a broken record) is left to the general kernel
+            if (!(e_area[e] > 0.0f && e_area[e] <= 1e20f && e_dist[e] > 0.0f && e_dist[e] <= 1e20f)) return 0;
+            nb[(size_t)a * 2 + deg[a]] = b; ne[(size_t)a * 2 + deg[a]++] = e;
+            nb[(size_t)b * 2 + deg[b]] = a; ne[(size_t)b * 2 + deg[b]++] = e;
+        }
+    // components in path order, each from its end with the lower device index
+    std::vector<uint32_t> order, edge, comp_beg;   // edge[k]: connection between order[k] and order[k + 1]
+    order.reserve(n); edge.reserve(n);
+    std::vector<uint8_t> seen(n, 0);
+    uint32_t longest = 0;
+    for (uint32_t r = 0; r < n; r++) {
+        if (seen[r] || deg[r] == 2) continue;
+        comp_beg.push_back((uint32_t)order.size());
+        for (uint32_t x = r, came = UINT32_MAX;;) {
+            seen[x] = 1;
+            order.push_back(x);
+            int k = -1;
+            for (int j = 0; j < deg[x]; j++) if (ne[(size_t)x * 2 + j] != came) k = j;
+            came = k < 0 ? UINT32_MAX : ne[(size_t)x * 2 + k];
+            edge.push_back(came);
+            if (k < 0) break;
+            x = nb[(size_t)x * 2 + k];
+        }
+        longest = std::max<uint32_t>(longest, (uint32_t)order.size() - comp_beg.back());
+    }
+    if (order.size() != n) return 0;   // a cycle has no end
+    comp_beg.push_back(n);
+    if (longest > 128) return 0;
+    auto warps = [&](uint32_t slots, std::vector<uint32_t>* first) {   // warps of `slots` slots; first[w]: its first position
+        uint32_t used = slots, w = 0;
+        for (size_t c = 0; c + 1 < comp_beg.size(); c++) {
+            const uint32_t sz = comp_beg[c + 1] - comp_beg[c];
+            if (used + sz > slots) {
+                w++;
+                used = 0;
+                if (first) first->push_back(comp_beg[c]);
+            }
+            used += sz;
+        }
+        if (first) first->push_back(n);
+        return w;
+    };
+    uint32_t R = longest <= 64 ? 2 : 4;
+    if (longest <= 32 && warps(32, nullptr) <= kPathThinWarps) R = 1;
+    std::vector<uint32_t> first;
+    const uint32_t W = warps(32 * R, &first);
+    pt_seg->assign((size_t)W * 32 * R, UINT32_MAX);
+    pt_area->assign(pt_seg->size(), 0.0f);
+    pt_dist->assign(pt_seg->size(), 1.0f);
+    parallel_for(W, [&](size_t w0, size_t w1) {
+        for (size_t w = w0; w < w1; w++)
+            for (uint32_t k = first[w]; k < first[w + 1]; k++) {
+                const size_t slot = (size_t)w * 32 * R + (k - first[w]);
+                const uint32_t x = order[k], e = edge[k];
+                const bool right_first = e != UINT32_MAX && ne[(size_t)x * 2] == e;
+                (*pt_seg)[slot] = x | (right_first ? 0x80000000u : 0u);
+                if (e == UINT32_MAX) continue;
+                (*pt_area)[slot] = e_area[e];
+                (*pt_dist)[slot] = e_dist[e];
+            }
+    }, 4096);
+    return R;
+}
+
+}  // namespace
+
 int build_network(const HostNet& hn, const Stimuli& stim, NetDev* dev, NetHost* host,
                   DeviceAllocs* allocs, const BuildOptions& opt) {
     const bool verbose = std::getenv("BNC_VERBOSE") != nullptr;
@@ -727,6 +816,11 @@ int build_network(const HostNet& hn, const Stimuli& stim, NetDev* dev, NetHost* 
         e_area[e] = area_conn;
         e_dist[e] = dist;
     }
+    // ---- unbranched networks: the slots of k_diffusion_path ----
+    std::vector<uint32_t> pt_seg;
+    std::vector<float> pt_area, pt_dist;
+    host->path_slots = opt.group_barriers ? path_layout(n, T, host->cluster, tile_seg_beg, tile_edge_beg, e_a, e_b, e_intra,
+                                                        e_area, e_dist, &pt_seg, &pt_area, &pt_dist) : 0;
     lap("edges");
     // incidence lists per device segment: the connections of its own tile that touch
     // it, in original connection order, a-role before b-role
@@ -1562,6 +1656,7 @@ int build_network(const HostNet& hn, const Stimuli& stim, NetDev* dev, NetHost* 
     int rc = BNC_OK;
     dev->n_seg = n; dev->n_tiles = T; dev->n_items = NI; dev->n_phases = n_phases;
     dev->n_syn = K; dev->n_rec = NR; dev->n_edges = E;
+    dev->n_pt = host->path_slots ? (uint32_t)(pt_seg.size() / (32 * host->path_slots)) : 0u;
     uint32_t flags = 0;
     if (!conn_ok.empty()) flags |= NF_DIFFUSION;
     if (aos.num_synapses > 0) flags |= NF_SYNAPSES;     // the reset keys on num_synapses, valid or not
@@ -1606,6 +1701,11 @@ int build_network(const HostNet& hn, const Stimuli& stim, NetDev* dev, NetHost* 
         dev->warp_seg = up(allocs, warp_seg, &rc);
         dev->warp_edge = up(allocs, warp_edge, &rc);
         dev->seg_edge = host->diff_gm ? up(allocs, seg_edge, &rc) : nullptr;
+        if (host->path_slots) {
+            dev->pt_seg = up(allocs, pt_seg, &rc);
+            dev->pt_area = up(allocs, pt_area, &rc);
+            dev->pt_dist = up(allocs, pt_dist, &rc);
+        }
         dev->e_a = up(allocs, e_a, &rc);
         dev->e_b = up(allocs, e_b, &rc);
         dev->e_intra = up(allocs, e_intra, &rc);

@@ -36,16 +36,9 @@ static __device__ __forceinline__ double dm_scale2(double p, int k) {
            __longlong_as_double((long long)(-54 + 1023) << 52);
 }
 
-BNC_MATH_FN double dm_exp(double x) {
-    if (x != x) return x;
-    if (x > 709.782712893384) return __longlong_as_double(0x7FF0000000000000ll);
-    if (x < -745.1332191019412) return 0.0;
-    const double LOG2E = 1.4426950408889634;
-    const double LN2_HI = 6.93147180369123816490e-01;
-    const double LN2_LO = 1.90821492927058770002e-10;
-    double kd = floor(x * LOG2E + 0.5);
-    double r = x - kd * LN2_HI;
-    r = r - kd * LN2_LO;
+// The Taylor polynomial of dm_exp on its reduced argument.  For |x| < 0.34 the reduction
+// leaves x as it is (k = 0), so dm_exp(x) is dm_exp_taylor(x).
+static __device__ __forceinline__ double dm_exp_taylor(double r) {
     double p = 1.0 / 6227020800.0;
     p = p * r + 1.0 / 479001600.0;
     p = p * r + 1.0 / 39916800.0;
@@ -60,6 +53,28 @@ BNC_MATH_FN double dm_exp(double x) {
     p = p * r + 0.5;
     p = p * r + 1.0;
     p = p * r + 1.0;
+    return p;
+}
+
+// dm_exp for |x| < 700: no special operands, and 2^k is a normal number.
+static __device__ __forceinline__ double dm_exp_mid(double x) {
+    const double kd = floor(x * 1.4426950408889634 + 0.5);
+    double r = x - kd * 6.93147180369123816490e-01;
+    r = r - kd * 1.90821492927058770002e-10;
+    return dm_exp_taylor(r) * __longlong_as_double((long long)((int)kd + 1023) << 52);
+}
+
+BNC_MATH_FN double dm_exp(double x) {
+    if (x != x) return x;
+    if (x > 709.782712893384) return __longlong_as_double(0x7FF0000000000000ll);
+    if (x < -745.1332191019412) return 0.0;
+    const double LOG2E = 1.4426950408889634;
+    const double LN2_HI = 6.93147180369123816490e-01;
+    const double LN2_LO = 1.90821492927058770002e-10;
+    double kd = floor(x * LOG2E + 0.5);
+    double r = x - kd * LN2_HI;
+    r = r - kd * LN2_LO;
+    const double p = dm_exp_taylor(r);
     return dm_scale2(p, (int)kd);
 }
 

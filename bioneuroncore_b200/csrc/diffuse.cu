@@ -9,8 +9,10 @@
 // sweep is a few independent shared-memory loads, the arithmetic and one barrier.
 // Every gather sums the segment's incident connections in original connection order,
 // the order of the reference's scatter loops, so results are bit-identical to them.
+#include <algorithm>
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
+#include <type_traits>
 #include "net.h"
 #include "physics.cuh"
 
@@ -347,6 +349,34 @@ __device__ __forceinline__ const double* residual_solve(const NetDev& d, const D
     return wa;
 }
 
+// The segment's step-1 current with its stimuli added: current steps
+// (simulation_host.cpp:189-209, 247-258: expiry, then add in order), then ramps
+// (simulation_host.cpp:261-276: the amplitude interpolated in FP32).
+__device__ __forceinline__ double stimulus_current(const NetDev& d, uint32_t g, double I, float dt,
+                                                   unsigned long long tick) {
+    if (d.cs_off) {
+        for (uint32_t k = d.cs_off[g]; k < d.cs_off[g + 1]; k++) {
+            if (!d.cs_alive[k]) continue;
+            unsigned long long dur = (unsigned long long)(d.cs_dur[k] / dt);
+            unsigned long long st0 = d.cs_start[k];
+            if (tick >= st0 + dur) { d.cs_alive[k] = 0; continue; }
+            if (tick >= st0 && tick < st0 + dur) I += d.cs_amp[k];
+        }
+    }
+    if (d.rp_off) {
+        for (uint32_t k = d.rp_off[g]; k < d.rp_off[g + 1]; k++) {
+            const unsigned long long st0 = d.rp_start[k], en = d.rp_end[k];
+            if (tick >= st0 && tick < en) {
+                const float frac = en > st0 ? (float)(tick - st0) / (float)(en - st0) : 1.0f;
+                const float a = d.rp_from[k];
+                const float amp = a + (d.rp_to[k] - a) * frac;
+                I += amp;
+            }
+        }
+    }
+    return I;
+}
+
 // Adds a warp's values to a per-CTA FP64 ledger slot (every thread of the CTA calls it).
 __device__ __forceinline__ void ledger_add(double* sh, int slot, double v) {
 #pragma unroll
@@ -400,29 +430,7 @@ k_diffusion(NetDev d, float dt, unsigned long long tick, uint32_t S, uint32_t E)
         float vf = (float)r->vol;
         if (vf < 1e-6f) vf = 1e-6f;
         t.vf[i] = vf;
-        // current stimuli (simulation_host.cpp:189-209, 247-258): expiry, then add in order
-        double I = r->itot;
-        if (d.cs_off) {
-            for (uint32_t k = d.cs_off[g]; k < d.cs_off[g + 1]; k++) {
-                if (!d.cs_alive[k]) continue;
-                unsigned long long dur = (unsigned long long)(d.cs_dur[k] / dt);
-                unsigned long long st0 = d.cs_start[k];
-                if (tick >= st0 + dur) { d.cs_alive[k] = 0; continue; }
-                if (tick >= st0 && tick < st0 + dur) I += d.cs_amp[k];
-            }
-        }
-        // ramps (simulation_host.cpp:261-276): the amplitude interpolated in FP32
-        if (d.rp_off) {
-            for (uint32_t k = d.rp_off[g]; k < d.rp_off[g + 1]; k++) {
-                const unsigned long long st0 = d.rp_start[k], en = d.rp_end[k];
-                if (tick >= st0 && tick < en) {
-                    const float frac = en > st0 ? (float)(tick - st0) / (float)(en - st0) : 1.0f;
-                    const float a = d.rp_from[k];
-                    const float amp = a + (d.rp_to[k] - a) * frac;
-                    I += amp;
-                }
-            }
-        }
+        const double I = stimulus_current(d, g, r->itot, dt, tick);
         t.itot[i] = I;
         d.ibuf[g] = I;
         t.incoff[i] = (uint16_t)(d.inc_off[g] - inc0);
@@ -1044,6 +1052,8 @@ k_diffusion(NetDev d, float dt, unsigned long long tick, uint32_t S, uint32_t E)
     }
 }
 
+#include "diffuse_path.cuh"
+
 size_t diffusion_smem_bytes(uint32_t max_segs, uint32_t max_edges) {
     return diff_layout(max_segs, max_edges, nullptr, nullptr);
 }
@@ -1114,6 +1124,7 @@ cudaError_t enqueue_diffusion(const NetDev& dev, const NetHost& host, float dt, 
         const cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) return e;
     }
+    if (host.path_slots && dev.diff_mode == 0u) return launch_diffusion_path(dev, host.path_slots, dt, tick, stream);
     const uint32_t S = host.max_tile_stride, E = host.max_tile_edges;
     const size_t smem = diffusion_smem_bytes(S, E);
     const uint32_t threads = std::max(host.diff_threads, diffusion_threads(host.max_tile_segs));

@@ -86,6 +86,15 @@ struct NetDev {
     // diffusion barrier groups (NetHost::diff_gm nonzero): per segment the tile-local
     // connection its thread handles (0xFFFF: none); null otherwise
     uint16_t* seg_edge;
+    // unbranched networks (NetHost::path_slots nonzero): 32 x path_slots slots per warp
+    // of k_diffusion_path, whole components laid end to end in path order.  Per slot its
+    // device segment (bit 31: the connection to the next slot comes before the one to the
+    // previous slot in connection order; UINT32_MAX: empty), and the contact area and
+    // length of the connection to the next slot (area 0: none)
+    uint32_t* pt_seg;         // [n_pt * 32 * path_slots] (nullptr otherwise)
+    float* pt_area;
+    float* pt_dist;
+    uint32_t n_pt;            // warps
     // edges (tile-grouped, tile-local endpoints)
     uint16_t* e_a;
     uint16_t* e_b;
@@ -268,6 +277,12 @@ constexpr double kMaxWarpTypes = 1.3;
 // matters more than divergence, and the requested depth is kept.
 constexpr uint32_t kAdaptiveFuseMinSegs = 1u << 16;
 
+// k_diffusion_path takes its low-latency form up to this many warps (4 per scheduler:
+// 1,800 warps 64.5 us against 72.8, 6,539 warps 172 against 169, 20,000 warps 544 against
+// 459), and one slot per lane up to one warp per scheduler.
+constexpr uint32_t kPathFewWarps = 2368;
+constexpr uint32_t kPathThinWarps = 592;
+
 // Host copy of everything the exporter needs to map device state back.
 struct NetHost {
     uint32_t n_seg = 0, n_conn = 0, n_syn_total = 0;
@@ -286,6 +301,7 @@ struct NetHost {
     uint32_t max_tile_stride = 0;            // own + ghost segments of the largest tile
     uint32_t cluster = 1;                    // CTAs per diffusion cluster (2: tiles in pairs)
     uint32_t diff_threads = 32;              // threads per diffusion CTA
+    uint32_t path_slots = 0;                 // slots per lane of k_diffusion_path (0: not an unbranched network)
     uint32_t diff_gm = 0;                    // diffusion barrier groups: 0 (CTA), 32 or 64 threads
     uint32_t group_tiles_32 = 0, group_tiles_64 = 0;   // tiles with warp / 64-thread barrier groups
     std::vector<uint32_t> phase_off;         // item range of each (chunk, phase) bucket (host copy)
