@@ -107,6 +107,140 @@ __device__ __forceinline__ double receptor_current(const RecKind& K, DMod& m, DS
     return I;
 }
 
+// What the receptor currents of one segment share through step 3 (V_m, the extracellular
+// ions and the volume are constant there): the GHK factors with their reciprocals, the
+// products of the constant side, NMDA's Mg2+ block.  A receptor's current depends on the
+// intracellular ions the receptor before it left, so a segment's receptors are one serial
+// chain, and its latency bounds the synapse step of any network that does not fill the
+// chip many times over.  With the reciprocals a receptor is about 16 dependent FP64
+// operations (9 cycles each) in place of three full divisions (112 cycles each) among 25,
+// and RecStep runs all four receptor kinds without divergence.
+struct RecSeg {
+    double A1, D1, y1, e1, o0, o1, o3;   // monovalent: out Na and K times e1, out Cl
+    double A2, D2, y2, o2;               // divalent: out Ca times e2
+    double cpm, yc;
+    float mg;
+    bool ok;                             // the fast form holds for this segment
+};
+
+__device__ __forceinline__ void rec_seg_fill(RecSeg& f, const DSeg& s, float dt) {
+    f.A1 = s.gc.A1; f.D1 = s.gc.D1; f.e1 = s.gc.e1;
+    f.A2 = s.gc.A2; f.D2 = s.gc.D2;
+    f.y1 = 1.0 / f.D1;
+    f.y2 = 1.0 / f.D2;
+    f.o0 = (double)s.out[0] * s.gc.e1;
+    f.o1 = (double)s.out[1] * s.gc.e1;
+    f.o2 = (double)s.out[2] * s.gc.e2;
+    f.o3 = (double)s.out[3];
+    f.cpm = FARADAY_CONST * s.vol / 1000.0;
+    f.yc = 1.0 / f.cpm;
+    f.mg = (float)(1.0f / (1.0f + (1.0f / 3.57f) * dm_exp(-0.062f * ((double)s.V))));
+    f.ok = s.gc.m1 == 0 && s.gc.m2 == 0 && fabs(f.cpm) >= 0x1p-100 && fabs(f.cpm) <= 0x1p100 && dt >= 1e-12f &&
+           dt <= 1e12f;
+}
+
+// A kind's constants as the step reads them (shared memory): permeabilities of its first
+// ion (Na, or Cl), K and Ca; time constants with their reciprocals rounded to nearest.
+struct RecK {
+    double P0, P1, P2, unused;
+    double rise, y_rise, decay, y_decay, des, y_des;
+};
+__device__ __forceinline__ void rec_k_fill(RecK& k, const RecKind& K) {
+    k.P0 = K.is_anion ? K.P_Cl : K.P_Na;
+    k.P1 = K.is_anion ? 0.0 : K.P_K;
+    k.P2 = K.nmda ? K.P_Ca : 0.0;
+    k.unused = 0.0;
+    k.rise = (double)K.tau_rise; k.y_rise = 1.0 / k.rise;
+    k.decay = (double)K.tau_decay; k.y_decay = 1.0 / k.decay;
+    k.des = K.tau_desens > 0.0f ? (double)K.tau_desens : 1.0; k.y_des = 1.0 / k.des;
+}
+
+// a / b rounded to nearest by Markstein's correction, given y = 1 / b rounded to nearest;
+// for a zero or away from under- and overflow (the callers see to that).
+__device__ __forceinline__ double rec_div(double a, double b, double y) {
+    const double q0 = a * y;
+    return __fma_rn(__fma_rn(-q0, b, a), y, q0);
+}
+// Zero, or of a magnitude in about [1e-200, 1e200], by the exponent field.
+__device__ __forceinline__ bool rec_in_range(double x) {
+    const uint32_t h = ((uint32_t)__double2hiint(x) & 0x7FFFFFFFu) - 0x16700000u;
+    return (h < 0x53000000u) | (x == 0.0);
+}
+// x + (to - x) dt / tau in float, clamped to [0, 1].  The float quotient is the binary64
+// one rounded again: that rounds twice to the same value (53 >= 2 x 24 + 2 bits), for
+// subnormal quotients of a decayed gate too.
+__device__ __forceinline__ float rec_relax(float x, float to, float dt, double tau, double ytau, bool& ok) {
+    const float a = (to - x) * dt;
+    ok &= fabsf(a) < 1e30f;
+    const float v = x + (float)rec_div((double)a, tau, ytau);
+    return v < 0.0f ? 0.0f : (v > 1.0f ? 1.0f : v);
+}
+__device__ __forceinline__ float rec_clamp(float x) { return x < 1e-9f ? 1e-9f : x; }
+
+// receptor_current for a default-conductance receptor of a segment whose RecSeg is ok, the
+// same operations in the same order; every lane of the warp takes part (`on`: this lane
+// has a receptor), so that lanes with different kinds run one instruction stream.  r_inf:
+// nt / (nt + EC50), also the desensitisation gate's target (K_desens is 0 for all kinds).
+// w: the desensitisation gate, for NMDA the inactivation gate.  Returns whether it holds;
+// nothing is changed in a lane where it does not (a value out of the range in which the
+// corrected quotients are the IEEE ones, or not finite).
+__device__ __forceinline__ bool receptor_step(const RecSeg& f, const RecK& K, int kind, bool on, float den, float area,
+                                              float& r, float& w, float (&in)[7], float dt, float r_inf, float mod_scale,
+                                              double& I) {
+    const bool an = kind >= 2, nmda = kind == 1;
+    bool ok = f.ok;
+    const bool up = r_inf > r;
+    const float rn = rec_relax(r, r_inf, dt, up ? K.rise : K.decay, up ? K.y_rise : K.y_decay, ok);
+    float wn = rec_relax(w, r_inf, dt, K.des, K.y_des, ok);
+    const float open = nmda ? rn : rn * (1.0f - wn);
+    const double N = (double)den * area;
+    const double n0 = an ? f.o3 - (double)in[3] * f.e1 : (double)in[0] - f.o0;
+    const double f0 = rec_div(f.A1 * n0, f.D1, f.y1);
+    const double f1 = rec_div(f.A1 * ((double)in[1] - f.o1), f.D1, f.y1);
+    const double I0 = K.P0 * f0 * N * open * mod_scale * A_TO_PA;
+    const double I1 = K.P1 * f1 * N * open * mod_scale * A_TO_PA;
+    const double q0 = rec_div(I0 * dt, f.cpm, f.yc);
+    const float c0 = rec_clamp((float)((double)(an ? in[3] : in[0]) - (an ? -q0 : q0)));
+    const float c1 = rec_clamp((float)((double)in[1] - rec_div(I1 * dt, f.cpm, f.yc)));
+    double It = an ? I0 : I0 + I1;
+    ok &= rec_in_range(I0) & (an | rec_in_range(I1));
+    float c2 = in[2];
+    if (__any_sync(0xFFFFFFFFu, on & nmda)) {
+        const double f2 = rec_div(f.A2 * ((double)in[2] - f.o2), f.D2, f.y2);
+        const double I2 = K.P2 * f2 * N * open * mod_scale * A_TO_PA;
+        if (nmda) {
+            It += I2;
+            ok &= rec_in_range(I2) & (fabsf(w) < 1e30f);
+            c2 = rec_clamp((float)((double)in[2] - 0.5 * rec_div(I2 * dt, f.cpm, f.yc)));
+            // dp_nmda_cdi_coagonist
+            const double Ca_uM = (double)c2 * MM_TO_UM;
+            const double cdi_inf = 1.0 - 0.8f * Ca_uM / (Ca_uM + 1.0f);
+            const bool fast = cdi_inf < (double)w;
+            wn = (float)((double)w + rec_div((cdi_inf - (double)w) * dt, fast ? 500.0 : 9000.0, fast ? 1.0 / 500.0 : 1.0 / 9000.0));
+            wn = wn < 0.0f ? 0.0f : (wn > 1.0f ? 1.0f : wn);
+            It = It * f.mg * ((double)wn * (10.0f / (10.0f + 1.0f)));
+        }
+    }
+    I = -It;
+    if (on && ok) {
+        r = rn;
+        w = wn;
+        if (an) in[3] = c0;
+        else { in[0] = c0; in[1] = c1; in[2] = c2; }
+    }
+    return ok;
+}
+
+// receptor_current out of line, for the receptors receptor_step does not hold for.
+struct RecSlow {
+    DMod m;
+    DSeg s;
+    double I;
+};
+__device__ __noinline__ void receptor_slow(RecSlow* x, int kind, float dt, float nt, float mod_scale) {
+    x->I = receptor_current(gRec[kind], x->m, x->s, dt, nt, mod_scale);
+}
+
 }  // namespace
 
 }  // namespace bnc

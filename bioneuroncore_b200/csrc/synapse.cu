@@ -9,7 +9,10 @@
 // the warp, since counts descend), and the j-th receptors of a slice's synapses are
 // adjacent, so the loads of a loop iteration are coalesced.  All four ionotropic
 // receptors run one code path with per-lane constants, so lanes holding different
-// receptor types do not serialise.  Presynaptic values come from the record the
+// receptor types do not serialise; a receptor's and a synapse's inputs are loaded one
+// step ahead.  What bounds the step is the latency of the longest chain of receptor
+// currents (55k segments: 16 synapses x 8 receptors, 1.2 us a receptor) and, when the
+// chip is full, instruction issue.  Presynaptic values come from the record the
 // diffusion kernel wrote after step 2.5 (V, Ca_out, the Cav2.1 gate).
 #include <cuda_runtime.h>
 #include "net.h"
@@ -236,9 +239,56 @@ __global__ void __launch_bounds__(256) k_release(NetDev d, float dt, unsigned lo
     if (rrp_max > 0.0f) d.sy_rrp[k] = rrp;
 }
 
+// One receptor's and one synapse's inputs, loaded one step ahead of their use: the
+// segment's chain of receptor currents then waits for arithmetic, not for loads.
+struct RecIn {
+    float den, s0, s1, s2;
+    uint8_t type, av;
+};
+__device__ __forceinline__ void rec_in_load(RecIn& x, const NetDev& d, uint32_t r) {
+    const size_t NR = d.n_rec;
+    x.type = d.rc_type[r];
+    x.av = d.rc_av[r];
+    x.den = d.rc_den[r];
+    x.s0 = d.rc_st[r];
+    x.s1 = d.rc_st[NR + r];
+    x.s2 = d.rc_st[2 * NR + r];
+}
+struct SynIn {
+    float cleft, parea, scale;
+    uint32_t n_rc, gjv;
+    uint8_t refr, sf;
+};
 template <bool kX>
-__global__ void __launch_bounds__(256, 4)
+__device__ __forceinline__ void syn_in_load(SynIn& x, const NetDev& d, uint32_t k, bool act) {
+    x.cleft = x.parea = x.scale = 0.0f;
+    x.n_rc = 0;
+    x.gjv = UINT32_MAX;
+    x.refr = x.sf = 0;
+    if (!act) return;
+    if (kX && d.sy_gj) x.gjv = d.sy_gj[k];   // a gap junction's side (simulation_host.cpp:373-402), else chemical
+    x.parea = d.sy_post_area[k];
+    x.scale = d.sy_scale[k];
+    if (!kX || x.gjv == UINT32_MAX) x.n_rc = d.rc_cnt[k];
+    if (!kX) {   // k_release ran the presynaptic half
+        x.sf = d.sy_flags[k];
+        x.cleft = d.sy_cleft[k];
+        x.refr = d.sy_refr[k];
+    }
+}
+
+// 64 threads a CTA spread the first warps, which hold the longest chains, over the SMs;
+// 128 registers hold the pipeline (1.28M segments, steps 3 and 4: 445 us at 8 CTAs per
+// SM, 493 at 6, 518 at 10; 55k segments: 156, 142, 209; 756 and 545 before the chain was
+// shortened and its loads moved a step ahead).
+constexpr unsigned kSynThreads = 64;
+
+template <bool kX>
+__global__ void __launch_bounds__(kSynThreads, 8)
 k_synapse(NetDev d, float dt, unsigned long long tick, int first_tick) {
+    __shared__ RecK rec_k[4];
+    if (threadIdx.x < 4) rec_k_fill(rec_k[threadIdx.x], gRec[threadIdx.x]);
+    __syncthreads();
     const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
     const uint32_t N = d.n_seg;
     const uint32_t lane = threadIdx.x & 31u;
@@ -263,7 +313,11 @@ k_synapse(NetDev d, float dt, unsigned long long tick, int first_tick) {
     float ecb_st = ecb_q != UINT32_MAX ? d.it_st[ecb_q] : 0.0f;
     double ib = valid ? d.ibuf[i] : 0.0;
     DSeg s;
+    RecSeg rs = {};
     s.V = valid ? d.V[i] : 0.0f;
+#pragma unroll
+    for (int q = 0; q < 7; q++) s.in[q] = 0.0f;
+    s.area = 0.0f;
     bool touched = false;
     if (cnt > 0) {
 #pragma unroll
@@ -275,6 +329,7 @@ k_synapse(NetDev d, float dt, unsigned long long tick, int first_tick) {
         s.area = d.area[i];
         s.vol = d.vol[i];
         ghk_cache_fill(s.gc, s.V);   // V_m is constant through step 3
+        rec_seg_fill(rs, s, dt);
     }
     const uint32_t K = d.n_syn;
     const uint32_t NR = d.n_rec;
@@ -283,26 +338,34 @@ k_synapse(NetDev d, float dt, unsigned long long tick, int first_tick) {
         base = d.w_off[t >> 5];
         rbase = d.rw_off[t >> 5];
     }
+    SynIn syn;
+    RecIn rec = {};
+    syn_in_load<kX>(syn, d, base + lane, cnt > 0);
+    {
+        const uint32_t has = __ballot_sync(0xFFFFFFFFu, syn.n_rc > 0);
+        if (syn.n_rc > 0) rec_in_load(rec, d, rbase + __popc(has & lt_mask));
+    }
     for (uint32_t kk = 0; kk < maxc; kk++) {
         const bool act = cnt > kk;
         const uint32_t n_act = __popc(__ballot_sync(0xFFFFFFFFu, act));
         const uint32_t k = base + lane;   // this lane's synapse in the slice (when act)
-        // a gap junction's side (simulation_host.cpp:373-402) or a chemical synapse
-        const uint32_t gjv = (kX && act && d.sy_gj) ? d.sy_gj[k] : UINT32_MAX;
+        const uint32_t gjv = syn.gjv;
         const bool chem = act && gjv == UINT32_MAX;
-        float cleft = 0.0f, cleft_e = 0.0f, rrp = 0.0f, rrp_max = 0.0f, bouton = 0.0f;
-        uint8_t refr = 0, sf = 0;
-        int ntt = 0;
-        uint32_t n_rc = 0;
+        float cleft = syn.cleft, cleft_e = 0.0f, rrp = 0.0f, rrp_max = 0.0f, bouton = 0.0f;
+        uint8_t refr = syn.refr, sf = syn.sf;
+        int ntt = sf >> 4;
+        const uint32_t n_rc = syn.n_rc;
+        const float post_area = syn.parea, scale = syn.scale;
+        syn_in_load<kX>(syn, d, k + n_act, cnt > kk + 1);   // the next synapse's
+        float spine = 0.0f, facil = 0.0f, camkii = 0.0f, calcn = 0.0f, weight = 0.0f, tauc = 1.0f;
         if (chem) {
-            if (kX) {
-                presyn_step<true>(d, k, K, tick, dt, cleft, cleft_e, rrp, rrp_max, bouton, refr, sf, ntt);
-            } else {   // k_release ran the presynaptic half
-                sf = d.sy_flags[k];
-                ntt = sf >> 4;
-                cleft = d.sy_cleft[k];
-                refr = d.sy_refr[k];
-            }
+            if (kX) presyn_step<true>(d, k, K, tick, dt, cleft, cleft_e, rrp, rrp_max, bouton, refr, sf, ntt);
+            spine = d.sy_spine[k];
+            facil = d.sy_facil[k];
+            camkii = d.sy_camkii[k];
+            calcn = d.sy_calcn[k];
+            weight = d.sy_weight[k];
+            tauc = d.sy_tauc[k];
             // NT into the postsynaptic segment (simulation_host.cpp:463-465)
             if (ntt == 0) nt_glu += cleft;
             else if (ntt == 1) nt_gaba += cleft;
@@ -320,34 +383,64 @@ k_synapse(NetDev d, float dt, unsigned long long tick, int first_tick) {
                 }
                 d.gl_cap[k] = cap;
             }
-            n_rc = d.rc_cnt[k];
         }
         // receptors (simulation_host.cpp:490-500), j-th receptors of the slice side by side
         float I_syn = 0.0f;
-        const float post_area = act ? d.sy_post_area[k] : 0.0f;
-        const float scale = act ? d.sy_scale[k] : 0.0f;
+        double I_rec = 0.0;
+        const float ri_ampa = nt_glu / (nt_glu + 0.5f), ri_nmda = nt_glu / (nt_glu + 1.0f),
+                    ri_gabaa = nt_gaba / (nt_gaba + 1.0f), ri_gly = nt_gly / (nt_gly + 0.5f);   // EC50 of each kind
         const uint32_t maxr = __reduce_max_sync(0xFFFFFFFFu, n_rc);
+        uint32_t has = __ballot_sync(0xFFFFFFFFu, n_rc > 0);
         for (uint32_t j = 0; j < maxr; j++) {
-            const uint32_t has = __ballot_sync(0xFFFFFFFFu, n_rc > j);
-            if (n_rc > j) {
-                const uint32_t r = rbase + __popc(has & lt_mask);
-                DMod m;
-                m.den = d.rc_den[r];
-                m.st[0] = d.rc_st[r];
-                m.st[1] = d.rc_st[(size_t)NR + r];
-                m.st[2] = d.rc_st[(size_t)2 * NR + r];
-                m.st[3] = m.st[4] = m.st[5] = m.st[6] = 0.0f;
-                m.area = (post_area > 0.0f) ? post_area : s.area;
-                m.av = d.rc_av[r];
-                const int kind = receptor_kind(d.rc_type[r]);
-                const float ntr = kind <= 1 ? nt_glu : (kind == 2 ? nt_gaba : nt_gly);
-                I_syn = (float)(I_syn + receptor_current(gRec[kind], m, s, dt, ntr, scale));
-                d.rc_st[r] = m.st[0];
-                d.rc_st[(size_t)NR + r] = m.st[1];
-                d.rc_st[(size_t)2 * NR + r] = m.st[2];
+            const uint32_t r = rbase + __popc(has & lt_mask);
+            rbase += __popc(has);
+            const RecIn cur = rec;
+            // the next receptor's: the synapse's, or the first of the next synapse
+            const bool last = j + 1 == maxr;
+            const uint32_t n_next = last ? syn.n_rc : n_rc;
+            const uint32_t has_next = __ballot_sync(0xFFFFFFFFu, n_next > (last ? 0u : j + 1));
+            if (n_next > (last ? 0u : j + 1)) rec_in_load(rec, d, rbase + __popc(has_next & lt_mask));
+            has = has_next;
+            const bool on = n_rc > j;
+            const int kind = receptor_kind(cur.type);
+            const float parea = (post_area > 0.0f) ? post_area : s.area;
+            float r0 = cur.s0, w0 = kind == 1 ? cur.s2 : cur.s1;   // the state words the kind updates
+            const bool held = receptor_step(rs, rec_k[kind], kind, on && cur.av == 0, cur.den, parea, r0, w0, s.in, dt,
+                                            kind == 0 ? ri_ampa : kind == 1 ? ri_nmda : kind == 2 ? ri_gabaa : ri_gly,
+                                            scale, I_rec);
+            if (on) {
+                if (held && cur.av == 0) {
+                    if (!touched) {   // dp_clamp_ions of the ions the receptor left alone
+#pragma unroll
+                        for (int q = 0; q < 7; q++) s.in[q] = rec_clamp(s.in[q]);
+                    }
+                    d.rc_st[r] = r0;
+                    d.rc_st[(size_t)(kind == 1 ? 2 : 1) * NR + r] = w0;
+                } else {
+                    RecSlow x;
+                    x.s = s;
+                    x.m.den = cur.den;
+                    x.m.st[0] = cur.s0;
+                    x.m.st[1] = cur.s1;
+                    x.m.st[2] = cur.s2;
+                    x.m.st[3] = x.m.st[4] = x.m.st[5] = x.m.st[6] = 0.0f;
+                    x.m.area = parea;
+                    x.m.av = cur.av;
+                    receptor_slow(&x, kind, dt, kind <= 1 ? nt_glu : (kind == 2 ? nt_gaba : nt_gly), scale);
+#pragma unroll
+                    for (int q = 0; q < 7; q++) s.in[q] = x.s.in[q];
+                    I_rec = x.I;
+                    d.rc_st[r] = x.m.st[0];
+                    d.rc_st[(size_t)NR + r] = x.m.st[1];
+                    d.rc_st[(size_t)2 * NR + r] = x.m.st[2];
+                }
+                I_syn = (float)(I_syn + I_rec);
                 touched = true;
             }
-            rbase += __popc(has);
+        }
+        if (maxr == 0) {   // no receptor in this slice: the next one's first is still to load
+            has = __ballot_sync(0xFFFFFFFFu, syn.n_rc > 0);
+            if (syn.n_rc > 0) rec_in_load(rec, d, rbase + __popc(has & lt_mask));
         }
         if (act && gjv != UINT32_MAX) {
             // gap junction (simulation_host.cpp:373-402): both sides compute the same
@@ -378,7 +471,6 @@ k_synapse(NetDev d, float dt, unsigned long long tick, int first_tick) {
         if (chem) {
             ib += I_syn;
             // spine Ca2+ (modifier_helpers.h:808-817)
-            float spine = d.sy_spine[k];
             {
                 float I_abs = I_syn < 0.0f ? -I_syn : I_syn;
                 float I_Ca = I_abs * 0.1f;
@@ -388,7 +480,7 @@ k_synapse(NetDev d, float dt, unsigned long long tick, int first_tick) {
                 if (spine < 0.0f) spine = 0.0f;
             }
             // clearance (simulation_host.cpp:505-510)
-            const auto clear_f = dm_exp(-dt / d.sy_tauc[k]);
+            const auto clear_f = dm_exp(-dt / tauc);
             if (!kX || !d.gl_cap) {   // with glia, they take glutamate, GABA and glycine instead
                 cleft *= clear_f;
                 if (cleft < 0.0f) cleft = 0.0f;
@@ -398,14 +490,12 @@ k_synapse(NetDev d, float dt, unsigned long long tick, int first_tick) {
                 if (cleft_e < 0.0f) cleft_e = 0.0f;
             }
             // BCM threshold, spine CaMKII/calcineurin, weight (simulation_host.cpp:527-576)
-            float facil = d.sy_facil[k];
             {
                 float Ca_uM = spine * 1000.0f;
                 float Ca_sq = Ca_uM * Ca_uM;
                 facil += (Ca_sq - facil) * dt / 300000.0f;
                 if (facil < 0.0f) facil = 0.0f;
             }
-            float camkii = d.sy_camkii[k], calcn = d.sy_calcn[k];
             {
                 float Ca_uM = spine * MM_TO_UM;
                 float Ca4 = Ca_uM * Ca_uM * Ca_uM * Ca_uM;
@@ -419,7 +509,6 @@ k_synapse(NetDev d, float dt, unsigned long long tick, int first_tick) {
                 if (calcn < 0.0f) calcn = 0.0f;
                 if (calcn > 1.0f) calcn = 1.0f;
             }
-            float weight = d.sy_weight[k];
             {
                 float dw = 0.0f;
                 if (camkii > 0.0f) dw += 0.0003f * camkii * dt;
@@ -537,10 +626,10 @@ uint32_t synapse_launches(const NetDev& dev) {
 cudaError_t launch_synapse(const NetDev& dev, float dt, unsigned long long tick, int first_tick,
                            cudaStream_t stream) {
     const bool extras = dev.syn_extras != 0;
-    if (extras) k_synapse<true><<<(dev.n_seg + 255) / 256, 256, 0, stream>>>(dev, dt, tick, first_tick);
+    if (extras) k_synapse<true><<<(dev.n_seg + kSynThreads - 1) / kSynThreads, kSynThreads, 0, stream>>>(dev, dt, tick, first_tick);
     else {
         if (dev.n_syn) k_release<<<(dev.n_syn + 255) / 256, 256, 0, stream>>>(dev, dt, tick);
-        k_synapse<false><<<(dev.n_seg + 255) / 256, 256, 0, stream>>>(dev, dt, tick, first_tick);
+        k_synapse<false><<<(dev.n_seg + kSynThreads - 1) / kSynThreads, kSynThreads, 0, stream>>>(dev, dt, tick, first_tick);
     }
     if (dev.gl_cap) k_glia<<<(dev.n_glia + 127) / 128, 128, 0, stream>>>(dev);
     if (dev.sy_gj) k_gj_commit<<<(dev.n_gj + 255) / 256 < 1184 ? (dev.n_gj + 255) / 256 : 1184, 256, 0, stream>>>(dev);
