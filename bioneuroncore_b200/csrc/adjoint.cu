@@ -336,6 +336,7 @@ __device__ inline double step1_seg(const AdjDev& d, const Ctx& c, const Lay& L, 
     s.atp = (kFull && d.has_atp) ? st[d.atp_w * Sm + i] : 0.0f;
     s.area = c.area;
     s.vol = c.vol;
+    dp_seg_derived(s);
     ghk_cache_fill(s.gc, s.V);
     double I_total = 0.0;
     const uint32_t ni = d.n_it[g];

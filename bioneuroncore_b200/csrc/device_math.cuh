@@ -56,15 +56,19 @@ static __device__ __forceinline__ double dm_exp_taylor(double r) {
     return p;
 }
 
-// dm_exp for |x| < 700: no special operands, and 2^k is a normal number.
+// dm_exp for |x| < 700: no special operands, and 2^k is a normal number.  The floor is the
+// downward-rounded addition of 1.5 x 2^52, whose low word is then k.
 static __device__ __forceinline__ double dm_exp_mid(double x) {
-    const double kd = floor(x * 1.4426950408889634 + 0.5);
+    const double big = 6755399441055744.0;
+    const double sh = __dadd_rd(x * 1.4426950408889634 + 0.5, big);
+    const double kd = sh - big;
     double r = x - kd * 6.93147180369123816490e-01;
     r = r - kd * 1.90821492927058770002e-10;
-    return dm_exp_taylor(r) * __longlong_as_double((long long)((int)kd + 1023) << 52);
+    return dm_exp_taylor(r) * __hiloint2double((__double2loint(sh) + 1023) << 20, 0);
 }
 
 BNC_MATH_FN double dm_exp(double x) {
+    if (((uint32_t)__double2hiint(x) & 0x7FFFFFFFu) < 0x4085E000u) return dm_exp_mid(x);   // |x| < 700
     if (x != x) return x;
     if (x > 709.782712893384) return __longlong_as_double(0x7FF0000000000000ll);
     if (x < -745.1332191019412) return 0.0;

@@ -66,7 +66,8 @@ __device__ __forceinline__ void rec_load(DSeg& s, const SegRec* r) {
     s.atp = r->atp;
     s.area = r->area;
     s.vol = r->vol;
-    ghk_cache_fill(s.gc, s.V);   // dead code for models without GHK currents
+    dp_seg_derived(s);            // these are dead code for models without such currents
+    ghk_cache_fill(s.gc, s.V);
 }
 
 __device__ __forceinline__ void rec_store(const DSeg& s, float v0, SegRec* r) {
@@ -169,8 +170,9 @@ k_phase(NetDev d, float dt, uint32_t b, uint32_t e) {
     if (type == 140) d.c21_cur[g] = make_float2(m.den, m.st[1]);
 }
 
-// run_item on a segment held in registers: the same models in the same order, the GHK
-// factors computed from the V the item starts with, as rec_load computes them.
+// run_item on a segment held in registers: the same models in the same order.  The
+// monovalent GHK factors are the group's (refilled when an item changed V), the divalent
+// ones, which few models read, computed from the V the item starts with.
 template <bool kDef, bool kX>
 __device__ __forceinline__ double run_item_s(uint8_t type, DMod& m, DSeg& s, float dt, float& glu, float gaba,
                                              float gly) {
@@ -178,7 +180,7 @@ __device__ __forceinline__ double run_item_s(uint8_t type, DMod& m, DSeg& s, flo
     switch (type) {
 #define BNC_ITEM(T, CALL)            \
     case T: {                        \
-        ghk_cache_fill(s.gc, s.V);   \
+        ghk_div_fill(s.gc, s.V);     \
         m.area = s.area;             \
         I = (CALL);                  \
         break;                       \
@@ -233,6 +235,12 @@ struct PhaseGroup {
 // arithmetic of the one-launch-per-phase path, so the results are the same bits.
 // The builder orders rows by (item count, item types), so a warp runs one sequence of
 // models; it forms groups only when no registered device modifier is present.
+// What bounds it: about 580 instructions per item (exponentials and divisions in binary64),
+// at 45% of issue slots behind the loads of the items' types and words.  Step 1 per tick at
+// 1.28M segments: 859 us at 4 CTAs per SM (64 registers), 914 at 3, 1,091 at 2, 933 at 5;
+// 1,007 before the models' divisions by a volume, a time constant or a GHK denominator
+// became corrected products (physics.cuh).  Items loaded one ahead cost more registers
+// than the waiting they saved (1,080 us).
 template <bool kX>
 __global__ void __launch_bounds__(256, BNC_GROUP_MIN_CTAS)
 k_phase_group(NetDev d, float dt, PhaseGroup grp) {
@@ -249,6 +257,8 @@ k_phase_group(NetDev d, float dt, PhaseGroup grp) {
     s.atp = r->atp;
     s.area = r->area;
     s.vol = r->vol;
+    dp_seg_derived(s);
+    ghk_mono_fill(s.gc, s.V);
     double itot = r->itot;
 #pragma unroll 1
     for (uint32_t j = 0; j < grp.n; j++) {
@@ -257,6 +267,7 @@ k_phase_group(NetDev d, float dt, PhaseGroup grp) {
         const uint32_t tf = d.it_tf[qi];
         const uint8_t type = (uint8_t)(tf & 0xFFu);
         const uint8_t fl = (uint8_t)(tf >> 8);
+        if (__float_as_uint(s.V) != __float_as_uint(s.gc.Vc)) ghk_mono_fill(s.gc, s.V);
         DMod m;
         m.den = d.it_den[qi];
         m.av = (fl & 2) ? (uint8_t)((fl >> 2) & 7) : (uint8_t)0;

@@ -14,6 +14,35 @@
 
 namespace bnc {
 
+// a / b rounded to nearest, given y = 1 / b rounded to nearest (Markstein's correction, 1990,
+// IBM J. Res. Dev. 34(1)): 27 cycles of latency against 112 for the division, and a third
+// of its instructions.  A NaN the correction makes of an infinite or zero-divided a * y is
+// put back.  Quotients under 2^-900, where the remainder would underflow, may be an ulp
+// off; every use adds the quotient to a float value, which that does not reach.
+__device__ __forceinline__ double dp_div_y(double a, double b, double y) {
+    const double q0 = a * y;
+    const double q = __fma_rn(__fma_rn(-q0, b, a), y, q0);
+    return q == q ? q : q0;
+}
+// a / c for a constant c: its reciprocal is folded at compile time.
+__device__ __forceinline__ double dp_over(double a, double c) { return dp_div_y(a, c, 1.0 / c); }
+
+// The same in binary32, for dividends that are zero or far from subnormal (a potential less
+// a constant).
+__device__ __forceinline__ float fp_over(float a, float c) {
+    const float y = 1.0f / c;
+    const float q0 = a * y;
+    const float q = __fmaf_rn(__fmaf_rn(-q0, c, a), y, q0);
+    return q == q ? q : q0;
+}
+// Over a value that is a constant in the default-parameter models only.
+template <bool kConst> __device__ __forceinline__ double dp_over_if(double a, double c) {
+    return kConst ? dp_over(a, c) : a / c;
+}
+template <bool kConst> __device__ __forceinline__ float fp_over_if(float a, float c) {
+    return kConst ? fp_over(a, c) : a / c;
+}
+
 // GHK factors that depend on V_m only.  V_m is constant while a segment's modifiers
 // (step 1) or a postsynaptic segment's receptors (step 3) run, so exp(-V_norm) and the
 // prefactor of run_tick_common.h:274-312 are evaluated once per segment and tick.  The
@@ -25,6 +54,7 @@ struct GhkCache {
     uint8_t m1, m2;    // branch: 0 general, 1 |V_norm| < 1e-6, 2 V_norm > 20, 3 V_norm < -20
     double A1, e1, D1; // monovalent/anion: k*F*V*0.001, exp(-V_norm), 1 - exp(-V_norm)
     double A2, e2, D2; // divalent
+    double y1;         // 1 / D1
 };
 
 // Segment state visible to a modifier while it runs (registers).
@@ -35,7 +65,12 @@ struct DSeg {
     float atp;
     float area;    // geometric membrane area, um^2 (run_tick_common.h:209-214)
     double vol;    // segment volume, um^3 (run_tick_common.h:262-266)
+    double ycpm;   // 1 / cpm(), set by dp_seg_derived
     GhkCache gc;
+    // charge per mole of the volume, FARADAY_CONST * vol / 1000.0
+    __device__ __forceinline__ double cpm() const;
+    // x / cpm()
+    __device__ __forceinline__ double over_cpm(double x) const;
 };
 
 // One modifier (or receptor) instance.  st[0..6] are the reference's state[0..6];
@@ -71,10 +106,18 @@ struct DMod {
 
 /* ---- helpers: reference include/run_tick_common.h, include/modifier_helpers.h ---- */
 
-/* modifier_helpers.h:1117-1121: arrays are double in the reference */
+__device__ __forceinline__ double DSeg::cpm() const { return dp_over(FARADAY_CONST * vol, 1000.0); }
+__device__ __forceinline__ double DSeg::over_cpm(double x) const { return dp_div_y(x, cpm(), ycpm); }
+__device__ __forceinline__ void dp_seg_derived(DSeg& s) { s.ycpm = 1.0 / s.cpm(); }
+// the extracellular share of a flux over cpm * EXTRA_VOLUME_RATIO is 4 x the one over cpm
+static_assert(EXTRA_VOLUME_RATIO == 0.25f, "a power of two");
+
+/* modifier_helpers.h:1117-1121: arrays are double in the reference (a float below 1e-9 in
+ * double is at most 1e-9f) */
 __device__ __forceinline__ void dp_clamp_ions(float* arr) {
+#pragma unroll
     for (int i = 0; i < 7; i++)
-        if ((double)arr[i] < 1e-9) arr[i] = (float)1e-9;
+        if (arr[i] < 1e-9f) arr[i] = 1e-9f;
 }
 /* run_tick_common.h:274-312 */
 static __device__ __forceinline__ double dp_ghk_mono(double V, double c_in, double c_out) {
@@ -104,21 +147,29 @@ static __device__ __forceinline__ double dp_ghk_anion(double V, double c_in, dou
 
 /* GHK with the per-segment factors (see GhkCache); identical results to
  * dp_ghk_mono/div/anion above. */
-static __device__ __forceinline__ void ghk_cache_fill(GhkCache& c, float Vf) {
+static __device__ __forceinline__ void ghk_mono_fill(GhkCache& c, float Vf) {
     double V = Vf;
     c.Vc = Vf;
-    double Vn1 = FARADAY_CONST * V * 0.001 / (GAS_CONST * CELSIUS_37);
+    double Vn1 = dp_over(FARADAY_CONST * V * 0.001, GAS_CONST * CELSIUS_37);
     c.m1 = (fabs(Vn1) < 1e-6) ? 1 : (Vn1 > 20.0) ? 2 : (Vn1 < -20.0) ? 3 : 0;
     double k1 = FARADAY_CONST / (GAS_CONST * CELSIUS_37);
     c.A1 = k1 * FARADAY_CONST * V * 0.001;
     c.e1 = (c.m1 == 0) ? dm_exp(-Vn1) : 0.0;
     c.D1 = 1.0 - c.e1;
-    double Vn2 = 2.0 * FARADAY_CONST * V * 0.001 / (GAS_CONST * CELSIUS_37);
+    c.y1 = 1.0 / c.D1;
+}
+static __device__ __forceinline__ void ghk_div_fill(GhkCache& c, float Vf) {
+    double V = Vf;
+    double Vn2 = dp_over(2.0 * FARADAY_CONST * V * 0.001, GAS_CONST * CELSIUS_37);
     c.m2 = (fabs(Vn2) < 1e-6) ? 1 : (Vn2 > 20.0) ? 2 : (Vn2 < -20.0) ? 3 : 0;
     double k2 = 4.0 * FARADAY_CONST / (GAS_CONST * CELSIUS_37);
     c.A2 = k2 * FARADAY_CONST * V * 0.001;
     c.e2 = (c.m2 == 0) ? dm_exp(-Vn2) : 0.0;
     c.D2 = 1.0 - c.e2;
+}
+static __device__ __forceinline__ void ghk_cache_fill(GhkCache& c, float Vf) {
+    ghk_mono_fill(c, Vf);
+    ghk_div_fill(c, Vf);
 }
 static __device__ __forceinline__ double dp_ghk_mono_c(const GhkCache& c, double V, double c_in, double c_out) {
     if ((float)V != c.Vc) return dp_ghk_mono(V, c_in, c_out);
@@ -126,7 +177,7 @@ static __device__ __forceinline__ double dp_ghk_mono_c(const GhkCache& c, double
         case 1: return FARADAY_CONST * (c_in - c_out);
         case 2: return c.A1 * c_in;
         case 3: return c.A1 * c_out;
-        default: return c.A1 * (c_in - c_out * c.e1) / c.D1;
+        default: return dp_div_y(c.A1 * (c_in - c_out * c.e1), c.D1, c.y1);
     }
 }
 static __device__ __forceinline__ double dp_ghk_div_c(const GhkCache& c, double V, double c_in, double c_out) {
@@ -144,7 +195,7 @@ static __device__ __forceinline__ double dp_ghk_anion_c(const GhkCache& c, doubl
         case 1: return FARADAY_CONST * (c_out - c_in);
         case 2: return c.A1 * c_out;
         case 3: return c.A1 * c_in;
-        default: return c.A1 * (c_out - c_in * c.e1) / c.D1;
+        default: return dp_div_y(c.A1 * (c_out - c_in * c.e1), c.D1, c.y1);
     }
 }
 
@@ -154,6 +205,13 @@ __device__ __forceinline__ double dp_ghk_P(float gamma_pS, float z, float cbar_m
     double z2F2 = z * z * FARADAY_CONST * FARADAY_CONST;
     double RT = GAS_CONST * CELSIUS_37;
     return gamma_S * RT / (z2F2 * cbar_mM);
+}
+// the same of a conductance that is not a constant
+__device__ __forceinline__ double dp_ghk_P_over(float gamma_pS, float z, float cbar_mM) {
+    double gamma_S = gamma_pS * PS_TO_S;
+    double z2F2 = z * z * FARADAY_CONST * FARADAY_CONST;
+    double RT = GAS_CONST * CELSIUS_37;
+    return dp_over(gamma_S * RT, z2F2 * cbar_mM);
 }
 /* modifier_helpers.h:58-66 */
 __device__ __forceinline__ void dp_nalcn_partial_P(float gamma_pS, double* P_Na, double* P_K, double* P_Ca) {
@@ -179,12 +237,14 @@ __device__ __forceinline__ float dp_nernst(float intra, float extra, float valen
 }
 /* modifier_helpers.h:132-135 */
 __device__ __forceinline__ float dp_vtrap(float x, float y) {
-    if (fabsf(x / y) < 1e-6f) return y * (1.0f - x / (2.0f * y));
-    return x / (1.0f - dm_exp(-x / y));
+    const float u = fp_over(x, y);
+    if (fabsf(u) < 1e-6f) return y * (1.0f - x / (2.0f * y));
+    return x / (1.0f - dm_exp(-u));
 }
 /* modifier_helpers.h:1090-1095 */
-__device__ __forceinline__ float dp_bz_act(float V, float vh, float k) { return 1.0f / (1.0f + dm_exp(-(V - vh) / k)); }
-__device__ __forceinline__ float dp_bz_inact(float V, float vh, float k) { return 1.0f / (1.0f + dm_exp((V - vh) / k)); }
+template <bool kConst = true>
+__device__ __forceinline__ float dp_bz_act(float V, float vh, float k) { return 1.0f / (1.0f + dm_exp(fp_over_if<kConst>(-(V - vh), k))); }
+__device__ __forceinline__ float dp_bz_inact(float V, float vh, float k) { return 1.0f / (1.0f + dm_exp(fp_over(V - vh, k))); }
 
 /* ---- gating helpers (modifier_helpers.h:145-215, 264-271, 468-472, 689-702, 1008-1018, 882-892, 909-913, 954-967, 1137-1170, 1188-1210) ---- */
 __device__ __forceinline__ float nav16_am(float V) { return 0.182f * dp_vtrap(V + 43.0f, 6.0f); }
@@ -193,7 +253,7 @@ __device__ __forceinline__ float nav16_ah(float V) { return 0.024f * dp_vtrap(V 
 __device__ __forceinline__ float nav16_bh(float V) { return 0.0091f * dp_vtrap(-(V + 75.0f), 5.0f); }
 __device__ __forceinline__ float nav16_m_inf(float V) { float a = nav16_am(V), b = nav16_bm(V); return a / (a + b); }
 __device__ __forceinline__ float nav16_m_tau(float V) { return 1.0f / (nav16_am(V) + nav16_bm(V)); }
-__device__ __forceinline__ float nav16_h_inf(float V) { return 1.0f / (1.0f + dm_exp((V + 72.0f) / 6.2f)); }
+__device__ __forceinline__ float nav16_h_inf(float V) { return 1.0f / (1.0f + dm_exp(fp_over(V + 72.0f, 6.2f))); }
 __device__ __forceinline__ float nav16_h_tau(float V) { return 1.0f / (nav16_ah(V) + nav16_bh(V)); }
 __device__ __forceinline__ float nav12_am(float V) { return 0.182f * dp_vtrap(V + 23.0f, 6.0f); }
 __device__ __forceinline__ float nav12_bm(float V) { return 0.124f * dp_vtrap(-(V + 23.0f), 6.0f); }
@@ -201,9 +261,9 @@ __device__ __forceinline__ float nav12_ah(float V) { return 0.024f * dp_vtrap(V 
 __device__ __forceinline__ float nav12_bh(float V) { return 0.0091f * dp_vtrap(-(V + 66.5f), 5.0f); }
 __device__ __forceinline__ float nav12_m_inf(float V) { float a = nav12_am(V), b = nav12_bm(V); return a / (a + b); }
 __device__ __forceinline__ float nav12_m_tau(float V) { return 1.0f / (nav12_am(V) + nav12_bm(V)); }
-__device__ __forceinline__ float nav12_h_inf(float V) { return 1.0f / (1.0f + dm_exp((V + 63.5f) / 6.2f)); }
+__device__ __forceinline__ float nav12_h_inf(float V) { return 1.0f / (1.0f + dm_exp(fp_over(V + 63.5f, 6.2f))); }
 __device__ __forceinline__ float nav12_h_tau(float V) { return 1.0f / (nav12_ah(V) + nav12_bh(V)); }
-__device__ __forceinline__ float cav21_m_inf(float V) { return 1.0f / (1.0f + dm_exp(-(V - -15.0f) / (6.0f + 1e-6f))); }
+__device__ __forceinline__ float cav21_m_inf(float V) { return 1.0f / (1.0f + dm_exp(fp_over(-(V - -15.0f), 6.0f + 1e-6f))); }
 __device__ __forceinline__ float cav21_h_inf(float V, float Ca_uM) {
     float h = 1.0f / (1.0f + dm_exp((V - -50.0f) / 8.0f));
     h *= 1.0f / (1.0f + Ca_uM / 3.0f);
@@ -217,17 +277,17 @@ __device__ __forceinline__ float cav31_h_tau(float V) {
 }
 __device__ __forceinline__ float cav31_m_tau(float V) {
     float dv = V - -20.0f;
-    float g = dm_exp(-(dv * dv) / (2.0f * 22.0f * 22.0f));
+    float g = dm_exp(fp_over(-(dv * dv), 2.0f * 22.0f * 22.0f));
     return 1.25f + (15.0f - 1.25f) * g;
 }
 __device__ __forceinline__ float kv_dr_m_tau(float V, float V_half) {
-    float tau = 14.6f * dm_exp(-(V - V_half) / 30.1f);
+    float tau = 14.6f * dm_exp(fp_over(-(V - V_half), 30.1f));
     if (tau < 0.3f) tau = 0.3f;
     if (tau > 200.0f) tau = 200.0f;
     return tau;
 }
 __device__ __forceinline__ float kir_f_open(float V) {
-    float Vn = (float)(FARADAY_CONST * V * 0.001f / (GAS_CONST * CELSIUS_37));
+    float Vn = (float)dp_over(FARADAY_CONST * V * 0.001f, GAS_CONST * CELSIUS_37);
     float Kd_Mg = 0.3f * dm_exp(-0.6f * 2.0f * Vn);
     float mg_block = 0.5f / Kd_Mg;
     float Kd_spm = 0.0775f * dm_exp(-0.5f * 4.0f * Vn);
@@ -242,7 +302,7 @@ __device__ __forceinline__ float sk_p_inf(float Ca) {
     return 1.0f / (1.0f + dm_pow(r, 4.0f));
 }
 __device__ __forceinline__ float bk_ha_po(float V_mV, float Ca) {
-    float Vn = (float)(FARADAY_CONST * V_mV * MV_TO_V / (GAS_CONST * CELSIUS_37));
+    float Vn = (float)dp_over(FARADAY_CONST * V_mV * MV_TO_V, GAS_CONST * CELSIUS_37);
     float J = 0.104f * dm_exp(0.55f * Vn);
     float L = 3.7e-8f * dm_exp(0.30f * Vn);
     if (Ca < 0.0f) Ca = 0.0f;
@@ -264,7 +324,7 @@ __device__ __forceinline__ float nak_pump_vnorm(float V_mV, float Na_i, float K_
     float atp = ATP_level;
     if (atp < 0.0f) atp = 0.0f;
     float f_ATP = atp / (atp + 0.5f);
-    float eta = (float)(0.8f * FARADAY_CONST * (V_mV * MV_TO_V) / (GAS_CONST * CELSIUS_37));
+    float eta = (float)dp_over(0.8f * FARADAY_CONST * (V_mV * MV_TO_V), GAS_CONST * CELSIUS_37);
     float a2 = 60.0f * dm_exp(0.5f * eta);
     float b2 = 6.0f * dm_exp(-(1.0f - 0.5f) * eta);
     float a1 = 200.0f * f_Na * f_ATP;
@@ -329,10 +389,8 @@ __device__ __forceinline__ double dp_nav_current(DMod& m, DSeg& s, float dt, int
     double flux = dp_ghk_mono_c(s.gc, V, ((double)s.in[0]), ((double)s.out[0]));
     double I_A = P_single * flux * (((double)m.den) * area) * open_prob;
     double I_Na = I_A * A_TO_PA;
-    double vol = s.vol;
-    double cpv = FARADAY_CONST * vol / 1000.0;
-    s.in[0] = (float)(((double)s.in[0]) - (I_Na * dt) / cpv);
-    s.out[0] = (float)(((double)s.out[0]) + (I_Na * dt) / (cpv * EXTRA_VOLUME_RATIO));
+    s.in[0] = (float)(((double)s.in[0]) - s.over_cpm(I_Na * dt));
+    s.out[0] = (float)(((double)s.out[0]) + 4.0 * s.over_cpm(I_Na * dt));
     dp_clamp_ions(s.in);
     dp_clamp_ions(s.out);
     return -I_Na;
@@ -346,14 +404,14 @@ __device__ __forceinline__ double dp_cav13_current(DMod& m, DSeg& s, float dt) {
     double Vhalf = ((kDef ? 0.0 : ((double)m.st[3])) != 0.0f) ? -fabs((kDef ? 0.0 : ((double)m.st[3]))) : -35.0f;
     double k = ((kDef ? 0.0 : ((double)m.st[4])) > 0.0f) ? (kDef ? 0.0 : ((double)m.st[4])) : 7.0f;
     double gamma_ps = ((kDef ? 0.0 : ((double)m.st[2])) > 0.0f) ? (kDef ? 0.0 : ((double)m.st[2])) : 25.0f;
-    float m_inf = (float)(1.0f / (1.0f + dm_exp(-(V - Vhalf) / (k + 1e-6f))));
+    float m_inf = (float)(1.0f / (1.0f + dm_exp(dp_over_if<kDef>(-(V - Vhalf), k + 1e-6f))));
     float tau_m = 2.0f;
     m.st[0] = (float)(((double)m.st[0]) + (m_inf - ((double)m.st[0])) * dt / tau_m);
     float Ca = (float)(((double)s.in[2]) * MM_TO_UM);
     float h_inf = 1.0f / (1.0f + dm_exp((V + 52.0f) / 8.0f));
     h_inf *= 1.0f / (1.0f + Ca / 3.0f);
     float tau_h = 100.0f;
-    m.st[1] = (float)(((double)m.st[1]) + (h_inf - ((double)m.st[1])) * dt / tau_h);
+    m.st[1] = (float)(((double)m.st[1]) + dp_over((h_inf - ((double)m.st[1])) * dt, tau_h));
     if (((double)m.st[0]) < 0.0f) m.st[0] = 0.0f;
     if (((double)m.st[1]) < 0.0f) m.st[1] = 0.0f;
     if (((double)m.st[0]) > 1.0f) m.st[0] = 1.0f;
@@ -365,10 +423,8 @@ __device__ __forceinline__ double dp_cav13_current(DMod& m, DSeg& s, float dt) {
     double flux = dp_ghk_div_c(s.gc, V, ca_in, ca_out);
     double I_A = P_single * flux * (((double)m.den) * area) * open_prob;
     double I_Ca = I_A * A_TO_PA;
-    double vol = s.vol;
-    double cpm = FARADAY_CONST * vol / 1000.0;
-    s.in[2] = (float)(((double)s.in[2]) - (I_Ca * dt) / (2.0f * cpm));
-    s.out[2] = (float)(((double)s.out[2]) - (I_Ca * dt) / (2.0f * cpm * EXTRA_VOLUME_RATIO));
+    s.in[2] = (float)(((double)s.in[2]) - 0.5 * s.over_cpm(I_Ca * dt));
+    s.out[2] = (float)(((double)s.out[2]) - 2.0 * s.over_cpm(I_Ca * dt));
     dp_clamp_ions(s.in);
     dp_clamp_ions(s.out);
     return -I_Ca;
@@ -381,7 +437,7 @@ __device__ __forceinline__ double dp_cav21_current(DMod& m, DSeg& s, float dt) {
     m.st[0] = (float)(((double)m.st[0]) + (m_inf - ((double)m.st[0])) * dt / 1.0f);
     float Ca = (float)(((double)s.in[2]) * MM_TO_UM);
     float h_inf = cav21_h_inf(V, Ca);
-    m.st[1] = (float)(((double)m.st[1]) + (h_inf - ((double)m.st[1])) * dt / 300.0f);
+    m.st[1] = (float)(((double)m.st[1]) + dp_over((h_inf - ((double)m.st[1])) * dt, 300.0f));
     if (((double)m.st[0]) < 0.0f) m.st[0] = 0.0f;
     if (((double)m.st[1]) < 0.0f) m.st[1] = 0.0f;
     if (((double)m.st[0]) > 1.0f) m.st[0] = 1.0f;
@@ -396,7 +452,7 @@ __device__ __forceinline__ double dp_nak_pump_current(DMod& m, DSeg& s, float dt
     double N = ((double)m.den) * area;
     float I_pump = (float)(N * v_norm * 75.0f * ELEMENTARY_CHARGE_C * A_TO_PA);
     float volume = (float)s.vol;
-    double cpm = FARADAY_CONST * volume / 1000.0;
+    double cpm = dp_over(FARADAY_CONST * volume, 1000.0);
     float transport = (float)(I_pump * dt / cpm);
     float na_avail = (float)((((double)s.in[0]) - 1e-9f) / 3.0f);
     float k_avail = (float)((((double)s.out[1]) - 1e-9f) * EXTRA_VOLUME_RATIO / 2.0f);
@@ -416,9 +472,9 @@ __device__ __forceinline__ double dp_nak_pump_current(DMod& m, DSeg& s, float dt
 }
 
 /* shared K-channel ion bookkeeping: intra K -= I*dt/cpv, extra K += .../EVR, clamp extra */
-__device__ __forceinline__ void dp_k_flux(DSeg& s, double I_K, float dt, double cpv) {
-    s.in[1] = (float)(((double)s.in[1]) - (I_K * dt) / cpv);
-    s.out[1] = (float)(((double)s.out[1]) + (I_K * dt) / (cpv * EXTRA_VOLUME_RATIO));
+__device__ __forceinline__ void dp_k_flux(DSeg& s, double I_K, float dt) {
+    s.in[1] = (float)(((double)s.in[1]) - s.over_cpm(I_K * dt));
+    s.out[1] = (float)(((double)s.out[1]) + 4.0 * s.over_cpm(I_K * dt));
     dp_clamp_ions(s.out);
 }
 
@@ -430,9 +486,9 @@ __device__ __forceinline__ double dp_kv42_current(DMod& m, DSeg& s, float dt) {
     double Vhalf = ((kDef ? 0.0 : ((double)m.st[4])) != 0.0f) ? -fabs((kDef ? 0.0 : ((double)m.st[4]))) : -10.0f;
     double k = ((kDef ? 0.0 : ((double)m.st[5])) > 0.0f) ? (kDef ? 0.0 : ((double)m.st[5])) : 13.5f;
     double gamma_ps = ((kDef ? 0.0 : ((double)m.st[2])) > 0.0f) ? (kDef ? 0.0 : ((double)m.st[2])) : 5.0f;
-    float m_inf = (float)(1.0f / (1.0f + dm_exp(-(V - Vhalf) / (k + 1e-6f))));
+    float m_inf = (float)(1.0f / (1.0f + dm_exp(dp_over_if<kDef>(-(V - Vhalf), k + 1e-6f))));
     float tau_m = 1.5f;
-    m.st[0] = (float)(((double)m.st[0]) + (m_inf - ((double)m.st[0])) * dt / tau_m);
+    m.st[0] = (float)(((double)m.st[0]) + dp_over((m_inf - ((double)m.st[0])) * dt, tau_m));
     float h_inf = 1.0f / (1.0f + dm_exp((V + 65.0f) / 8.0f));
     float tau_h = kv42_h_tau(V);
     m.st[1] = (float)(((double)m.st[1]) + (h_inf - ((double)m.st[1])) * dt / tau_h);
@@ -441,20 +497,18 @@ __device__ __forceinline__ double dp_kv42_current(DMod& m, DSeg& s, float dt) {
     if (((double)m.st[0]) > 1.0f) m.st[0] = 1.0f;
     if (((double)m.st[1]) > 1.0f) m.st[1] = 1.0f;
     float camkii = 0.0f;   /* no CaMKII modifiers in supported networks */
-    m.st[3] = (float)(((double)m.st[3]) + (camkii * 0.5f - ((double)m.st[3])) * dt / 5000.0f);
+    m.st[3] = (float)(((double)m.st[3]) + dp_over((camkii * 0.5f - ((double)m.st[3])) * dt, 5000.0f));
     if (((double)m.st[3]) < 0.0f) m.st[3] = 0.0f;
     if (((double)m.st[3]) > 1.0f) m.st[3] = 1.0f;
     double gamma_eff = gamma_ps * (1.0f - ((double)m.st[3]) * 0.7f);
     float K_i = s.in[1];
     float K_o = s.out[1];
-    double P_single = dp_ghk_P((float)gamma_eff, 1.0f, GHK_CBAR_K_MM);
+    double P_single = dp_ghk_P_over((float)gamma_eff, 1.0f, GHK_CBAR_K_MM);
     double open_prob = ((double)m.st[0]) * ((double)m.st[0]) * ((double)m.st[0]) * ((double)m.st[1]);
     double flux = dp_ghk_mono_c(s.gc, V, K_i, K_o);
     double I_A = P_single * flux * (((double)m.den) * area) * open_prob;
     double I_K = I_A * A_TO_PA;
-    double vol = s.vol;
-    double cpv = FARADAY_CONST * vol / 1000.0;
-    dp_k_flux(s, I_K, dt, cpv);
+    dp_k_flux(s, I_K, dt);
     return -I_K;
 }
 
@@ -464,14 +518,14 @@ __device__ __forceinline__ double dp_kv31_current(DMod& m, DSeg& s, float dt) {
     float V = s.V;
     float area = m.area;
     float Vhalf = 10.0f, k = 10.0f, gamma_ps = 27.0f;
-    float m_inf = 1.0f / (1.0f + dm_exp(-(V - Vhalf) / (k + 1e-6f)));
+    float m_inf = 1.0f / (1.0f + dm_exp(fp_over(-(V - Vhalf), k + 1e-6f)));
     float tau_m = 1.0f;
     m.st[0] = (float)(((double)m.st[0]) + (m_inf - ((double)m.st[0])) * dt / tau_m);
     if (((double)m.st[0]) < 0.0f) m.st[0] = 0.0f;
     if (((double)m.st[0]) > 1.0f) m.st[0] = 1.0f;
-    float h_inf = 1.0f / (1.0f + dm_exp((V + 30.0f) / 6.0f));
+    float h_inf = 1.0f / (1.0f + dm_exp(fp_over(V + 30.0f, 6.0f)));
     float tau_h = 2000.0f;
-    m.st[1] = (float)(((double)m.st[1]) + (h_inf - ((double)m.st[1])) * dt / tau_h);
+    m.st[1] = (float)(((double)m.st[1]) + dp_over((h_inf - ((double)m.st[1])) * dt, tau_h));
     if (((double)m.st[1]) < 0.0f) m.st[1] = 0.0f;
     if (((double)m.st[1]) > 1.0f) m.st[1] = 1.0f;
     float K_i = s.in[1];
@@ -490,9 +544,7 @@ __device__ __forceinline__ double dp_kv31_current(DMod& m, DSeg& s, float dt) {
     double flux = dp_ghk_mono_c(s.gc, V, K_i, K_o);
     double I_A = P_single * flux * (((double)m.den) * area) * open_prob;
     double I_K = I_A * A_TO_PA;
-    double vol = s.vol;
-    double cpv = FARADAY_CONST * vol / 1000.0;
-    dp_k_flux(s, I_K, dt, cpv);
+    dp_k_flux(s, I_K, dt);
     return -I_K;
 }
 
@@ -508,9 +560,10 @@ __device__ __forceinline__ double dp_cav31_current(DMod& m, DSeg& s, float dt) {
     float tau_m = cav31_m_tau(V);
     float tau_h = cav31_h_tau(V);
     float sub_dt = dt / 10.0f;
+    const double tm = tau_m, th = tau_h, ym = 1.0 / tm, yh = 1.0 / th;
     for (int step = 0; step < 10; step++) {
-        m_val += (m_inf - m_val) * sub_dt / tau_m;
-        h_val += (h_inf - h_val) * sub_dt / tau_h;
+        m_val += dp_div_y((m_inf - m_val) * sub_dt, tm, ym);
+        h_val += dp_div_y((h_inf - h_val) * sub_dt, th, yh);
     }
     if (m_val < 0.0f) m_val = 0.0f;
     if (m_val > 1.0f) m_val = 1.0f;
@@ -530,7 +583,7 @@ __device__ __forceinline__ double dp_cav31_current(DMod& m, DSeg& s, float dt) {
     double I_A = P_single * flux * (((double)m.den) * area) * open_prob;
     double I_CaT = I_A * A_TO_PA;
     float volume = (float)s.vol;
-    float charge_per_mole = (float)(FARADAY_CONST * volume / 1000.0);
+    float charge_per_mole = (float)dp_over(FARADAY_CONST * volume, 1000.0);
     s.in[2] = (float)(((double)s.in[2]) - (I_CaT * dt) / (2.0f * charge_per_mole));
     return -I_CaT;
 }
@@ -551,7 +604,7 @@ __device__ __forceinline__ double dp_pmca_current(DMod& m, DSeg& s, float dt) {
     double N = ((double)m.den) * area;
     float I_pump = (float)(N * 100.0f * f_Ca * f_ATP * ELEMENTARY_CHARGE_C * 2.0f * A_TO_PA);
     float volume = (float)s.vol;
-    double cpv = FARADAY_CONST * volume / 1000.0;
+    double cpv = dp_over(FARADAY_CONST * volume, 1000.0);
     float transport = (float)(I_pump * dt / (2.0f * cpv));
     float ca_avail = (float)(((double)s.in[2]) - 1e-9f);
     if (ca_avail < 0.0f) ca_avail = 0.0f;
@@ -575,7 +628,7 @@ __device__ __forceinline__ double dp_ncx_current(DMod& m, DSeg& s, float dt) {
     double N = ((double)m.den) * area;
     float I_ncx = (float)(N * 500.0f * flux_norm * ELEMENTARY_CHARGE_C * A_TO_PA);
     float volume = (float)s.vol;
-    double cpv = FARADAY_CONST * volume / 1000.0;
+    double cpv = dp_over(FARADAY_CONST * volume, 1000.0);
     float transport = (float)(I_ncx * dt / cpv);
     if (transport > Ca_i) transport = Ca_i;
     if (transport < -Na_i / 3.0f) transport = -Na_i / 3.0f;
@@ -681,10 +734,8 @@ __device__ __forceinline__ double dp_sk_current(DMod& m, DSeg& s, float dt) {
     double flux = dp_ghk_mono_c(s.gc, V, K_i, K_o);
     double I_A = P_single * flux * (((double)m.den) * area) * open_prob;
     float I_K = (float)(I_A * A_TO_PA);
-    double vol = s.vol;
-    double cpv = FARADAY_CONST * vol / 1000.0f;
-    s.in[1] = (float)(((double)s.in[1]) - (I_K * dt) / cpv);
-    s.out[1] = (float)(((double)s.out[1]) + (I_K * dt) / (cpv * EXTRA_VOLUME_RATIO));
+    s.in[1] = (float)(((double)s.in[1]) - s.over_cpm(I_K * dt));
+    s.out[1] = (float)(((double)s.out[1]) + 4.0 * s.over_cpm(I_K * dt));
     dp_clamp_ions(s.out);
     return -I_K;
 }
@@ -708,10 +759,8 @@ __device__ __forceinline__ double dp_bk_current(DMod& m, DSeg& s, float dt) {
     double flux = dp_ghk_mono_c(s.gc, V, K_i, K_o);
     double I_A = P_single * flux * (((double)m.den) * area) * open_prob;
     float I_K = (float)(I_A * A_TO_PA);
-    double vol = s.vol;
-    double cpv = FARADAY_CONST * vol / 1000.0f;
-    s.in[1] = (float)(((double)s.in[1]) - (I_K * dt) / cpv);
-    s.out[1] = (float)(((double)s.out[1]) + (I_K * dt) / (cpv * EXTRA_VOLUME_RATIO));
+    s.in[1] = (float)(((double)s.in[1]) - s.over_cpm(I_K * dt));
+    s.out[1] = (float)(((double)s.out[1]) + 4.0 * s.over_cpm(I_K * dt));
     dp_clamp_ions(s.out);
     return -I_K;
 }
@@ -727,8 +776,8 @@ __device__ __forceinline__ double dp_nap_current(DMod& m, DSeg& s, float dt) {
     double gamma_ps = ((kDef ? 0.0 : ((double)m.st[3])) > 0.0f) ? (kDef ? 0.0 : ((double)m.st[3])) : 20.7f;
     double tau_m = ((kDef ? 0.0 : ((double)m.st[4])) > 0.0f) ? (kDef ? 0.0 : ((double)m.st[4])) : 5.0f;
     double Po = ((kDef ? 0.0 : ((double)m.st[5])) > 0.0f) ? (kDef ? 0.0 : ((double)m.st[5])) : 0.016f;
-    float m_inf = dp_bz_act(V, (float)V_half, (float)k_m);
-    m_val += (m_inf - m_val) * dt / tau_m;
+    float m_inf = dp_bz_act<kDef>(V, (float)V_half, (float)k_m);
+    m_val += dp_over_if<kDef>((m_inf - m_val) * dt, tau_m);
     if (m_val < 0.0f) m_val = 0.0f;
     if (m_val > 1.0f) m_val = 1.0f;
     m.st[0] = (float)m_val;
@@ -737,9 +786,7 @@ __device__ __forceinline__ double dp_nap_current(DMod& m, DSeg& s, float dt) {
     double flux = dp_ghk_mono_c(s.gc, V, Na_i, Na_o);
     double I_A = P_single * flux * (((double)m.den) * area) * (m_val * Po);
     float I_Na = (float)(I_A * A_TO_PA);
-    double vol = s.vol;
-    double cpv = FARADAY_CONST * vol / 1000.0f;
-    s.in[0] = (float)(((double)s.in[0]) - (I_Na * dt) / cpv);
+    s.in[0] = (float)(((double)s.in[0]) - s.over_cpm(I_Na * dt));
     dp_clamp_ions(s.in);
     return -I_Na;
 }
@@ -756,9 +803,7 @@ __device__ __forceinline__ double dp_kir_current(DMod& m, DSeg& s, float dt) {
     double flux = dp_ghk_mono_c(s.gc, V, K_i, K_o);
     double I_A = P_single * flux * (((double)m.den) * area) * f_open;
     double I_K = I_A * A_TO_PA;
-    double vol = s.vol;
-    double cpv = FARADAY_CONST * vol / 1000.0f;
-    dp_k_flux(s, I_K, dt, cpv);
+    dp_k_flux(s, I_K, dt);
     return -I_K;
 }
 
@@ -775,9 +820,7 @@ __device__ __forceinline__ double dp_k2p_current(DMod& m, DSeg& s, float dt) {
     double flux = dp_ghk_mono_c(s.gc, V, K_i, K_o);
     double I_A = P_single * flux * (((double)m.den) * area) * Po;
     double I_K = I_A * A_TO_PA;
-    double vol = s.vol;
-    double cpv = FARADAY_CONST * vol / 1000.0;
-    dp_k_flux(s, I_K, dt, cpv);
+    dp_k_flux(s, I_K, dt);
     return -I_K;
 }
 
@@ -792,7 +835,7 @@ __device__ __forceinline__ double dp_kv7_current(DMod& m, DSeg& s, float dt) {
     double tau_act = ((kDef ? 0.0 : ((double)m.st[4])) > 0.0f) ? (kDef ? 0.0 : ((double)m.st[4])) : 100.0f;
     double tau_deact = ((kDef ? 0.0 : ((double)m.st[5])) > 0.0f) ? (kDef ? 0.0 : ((double)m.st[5])) : 60.0f;
     double pip2 = ((kDef ? 1.0 : ((double)m.st[6])) >= 0.0f) ? (kDef ? 1.0 : ((double)m.st[6])) : 1.0f;
-    float m_inf = (float)(1.0f / (1.0f + dm_exp(-(V - V_half) / k_slope)));
+    float m_inf = (float)(1.0f / (1.0f + dm_exp(dp_over_if<kDef>(-(V - V_half), k_slope))));
     float tau_m = (float)(tau_deact + (tau_act - tau_deact) * m_inf);
     if (tau_m < 1.0f) tau_m = 1.0f;
     m_val += (m_inf - m_val) * dt / tau_m;
@@ -809,9 +852,7 @@ __device__ __forceinline__ double dp_kv7_current(DMod& m, DSeg& s, float dt) {
     double flux = dp_ghk_mono_c(s.gc, V, K_i, K_o);
     double I_A = P_single * flux * (((double)m.den) * area) * (m_val * pip2 * pkc_suppress);
     double I_K = I_A * A_TO_PA;
-    double vol = s.vol;
-    double cpv = FARADAY_CONST * vol / 1000.0;
-    dp_k_flux(s, I_K, dt, cpv);
+    dp_k_flux(s, I_K, dt);
     return -I_K;
 }
 
@@ -824,7 +865,7 @@ __device__ __forceinline__ double dp_kvdr_current(DMod& m, DSeg& s, float dt) {
     double V_half = ((kDef ? 0.0 : ((double)m.st[1])) != 0.0f) ? (kDef ? 0.0 : ((double)m.st[1])) : -30.0f;
     double k = ((kDef ? 0.0 : ((double)m.st[2])) > 0.0f) ? (kDef ? 0.0 : ((double)m.st[2])) : 6.0f;
     double tau = ((kDef ? 0.0 : ((double)m.st[4])) > 0.0f) ? (kDef ? 0.0 : ((double)m.st[4])) : kv_dr_m_tau(V, (float)V_half);
-    float m_inf = (float)(1.0f / (1.0f + dm_exp(-(V - V_half) / (k + 1e-6f))));
+    float m_inf = (float)(1.0f / (1.0f + dm_exp(dp_over_if<kDef>(-(V - V_half), k + 1e-6f))));
     m_val += (m_inf - m_val) * dt / (tau + 1e-6f);
     if (m_val < 0.0f) m_val = 0.0f;
     if (m_val > 1.0f) m_val = 1.0f;
@@ -835,10 +876,10 @@ __device__ __forceinline__ double dp_kvdr_current(DMod& m, DSeg& s, float dt) {
     double flux = dp_ghk_mono_c(s.gc, V, K_i, K_o);
     double I_A = P_single * flux * (((double)m.den) * area) * m_val;
     double I_K = I_A * A_TO_PA;
-    double vol = s.vol;
-    float charge_per_mole_vol = (float)(FARADAY_CONST * vol / 1000.0);
-    s.in[1] = (float)(((double)s.in[1]) - (I_K * dt) / charge_per_mole_vol);
-    s.out[1] = (float)(((double)s.out[1]) + (I_K * dt) / (charge_per_mole_vol * EXTRA_VOLUME_RATIO));
+    float charge_per_mole_vol = (float)s.cpm();
+    const double dK = (I_K * dt) / charge_per_mole_vol;
+    s.in[1] = (float)(((double)s.in[1]) - dK);
+    s.out[1] = (float)(((double)s.out[1]) + 4.0 * dK);
     dp_clamp_ions(s.in);
     dp_clamp_ions(s.out);
     return -I_K;
@@ -857,8 +898,8 @@ __device__ __forceinline__ double dp_hcn1_current(DMod& m, DSeg& s, float dt) {
     float camp = 0.1f;  /* segment_camp_um: no cAMP/PKA modifier -> basal 0.1 uM (units.h:324) */
     float Ve = V_half + 15.0f * camp / (camp + 0.5f);
     float mv = m.st[0];
-    float mi = 1.0f / (1.0f + dm_exp(((float)V - Ve) / k));
-    float tau_eff = (V < Ve) ? (float)(tau_open * dm_exp((V - Ve) / 15.0f)) : tau_close;
+    float mi = 1.0f / (1.0f + dm_exp(fp_over_if<kDef>((float)V - Ve, k)));
+    float tau_eff = (V < Ve) ? (float)(tau_open * dm_exp(dp_over(V - Ve, 15.0f))) : tau_close;
     mv += (mi - mv) * dt / tau_eff;
     if (mv < 0.0f) mv = 0.0f;
     if (mv > 1.0f) mv = 1.0f;
@@ -870,12 +911,10 @@ __device__ __forceinline__ double dp_hcn1_current(DMod& m, DSeg& s, float dt) {
     double flux_K = dp_ghk_mono_c(s.gc, V, ((double)s.in[1]), ((double)s.out[1]));
     double In = P_Na * flux_Na * N * mv * A_TO_PA;
     double Ik = P_K * flux_K * N * mv * A_TO_PA;
-    double vol = s.vol;
-    double cpm = FARADAY_CONST * vol / 1000.0;
-    s.in[0] = (float)(((double)s.in[0]) - (In * dt) / cpm);
-    s.in[1] = (float)(((double)s.in[1]) - (Ik * dt) / cpm);
-    s.out[0] = (float)(((double)s.out[0]) + (In * dt) / (cpm * EXTRA_VOLUME_RATIO));
-    s.out[1] = (float)(((double)s.out[1]) + (Ik * dt) / (cpm * EXTRA_VOLUME_RATIO));
+    s.in[0] = (float)(((double)s.in[0]) - s.over_cpm(In * dt));
+    s.in[1] = (float)(((double)s.in[1]) - s.over_cpm(Ik * dt));
+    s.out[0] = (float)(((double)s.out[0]) + 4.0 * s.over_cpm(In * dt));
+    s.out[1] = (float)(((double)s.out[1]) + 4.0 * s.over_cpm(Ik * dt));
     dp_clamp_ions(s.in);
     dp_clamp_ions(s.out);
     return -(In + Ik);
@@ -893,14 +932,12 @@ __device__ __forceinline__ double dp_nalcn_current(DMod& m, DSeg& s, float dt) {
     float Ina = (float)(P_Na * dp_ghk_mono_c(s.gc, V, ((double)s.in[0]), ((double)s.out[0])) * N * A_TO_PA);
     float Ik = (float)(P_K * dp_ghk_mono_c(s.gc, V, ((double)s.in[1]), ((double)s.out[1])) * N * A_TO_PA);
     float Ica = (float)(P_Ca * dp_ghk_div_c(s.gc, V, ((double)s.in[2]), ((double)s.out[2])) * N * A_TO_PA);
-    double vol = s.vol;
-    double cpm = FARADAY_CONST * vol / 1000.0;
-    s.in[0] = (float)(((double)s.in[0]) - (Ina * dt) / cpm);
-    s.in[1] = (float)(((double)s.in[1]) - (Ik * dt) / cpm);
-    s.in[2] = (float)(((double)s.in[2]) - (Ica * dt) / (2.0f * cpm));
-    s.out[0] = (float)(((double)s.out[0]) + (Ina * dt) / (cpm * EXTRA_VOLUME_RATIO));
-    s.out[1] = (float)(((double)s.out[1]) + (Ik * dt) / (cpm * EXTRA_VOLUME_RATIO));
-    s.out[2] = (float)(((double)s.out[2]) + (Ica * dt) / (2.0f * cpm * EXTRA_VOLUME_RATIO));
+    s.in[0] = (float)(((double)s.in[0]) - s.over_cpm(Ina * dt));
+    s.in[1] = (float)(((double)s.in[1]) - s.over_cpm(Ik * dt));
+    s.in[2] = (float)(((double)s.in[2]) - 0.5 * s.over_cpm(Ica * dt));
+    s.out[0] = (float)(((double)s.out[0]) + 4.0 * s.over_cpm(Ina * dt));
+    s.out[1] = (float)(((double)s.out[1]) + 4.0 * s.over_cpm(Ik * dt));
+    s.out[2] = (float)(((double)s.out[2]) + 2.0 * s.over_cpm(Ica * dt));
     dp_clamp_ions(s.in);
     dp_clamp_ions(s.out);
     return -(Ina - Ik + Ica);
@@ -914,8 +951,6 @@ __device__ __forceinline__ double dp_ionotropic(DMod& m, DSeg& s, float dt, floa
                             float mod_scale) {
     float area = m.area;
     double V = ((double)s.V);
-    double vol = s.vol;
-    double cpm = FARADAY_CONST * vol / 1000.0;
     float p_gamma_ps = gamma_ps;
     if (!kDef) {
         float stav = (m.av == 7) ? m.area : ((m.av > 0 && m.av < 7) ? m.st[m.av] : 0.0f);
@@ -944,7 +979,7 @@ __device__ __forceinline__ double dp_ionotropic(DMod& m, DSeg& s, float dt, floa
         double P_Cl = dp_ghk_P(p_gamma_ps, 1.0f, GHK_CBAR_CL_MM);
         double flux_Cl = dp_ghk_anion_c(s.gc, V, ((double)s.in[3]), ((double)s.out[3]));
         double I_Cl = P_Cl * flux_Cl * N * open_prob * mod_scale * A_TO_PA;
-        s.in[3] = (float)(((double)s.in[3]) + (I_Cl * dt) / cpm);
+        s.in[3] = (float)(((double)s.in[3]) + s.over_cpm(I_Cl * dt));
         dp_clamp_ions(s.in);
         return -I_Cl;
     }
@@ -953,12 +988,12 @@ __device__ __forceinline__ double dp_ionotropic(DMod& m, DSeg& s, float dt, floa
     double I_Na = P_Na * dp_ghk_mono_c(s.gc, V, ((double)s.in[0]), ((double)s.out[0])) * N * open_prob * mod_scale * A_TO_PA;
     double I_K = P_K * dp_ghk_mono_c(s.gc, V, ((double)s.in[1]), ((double)s.out[1])) * N * open_prob * mod_scale * A_TO_PA;
     I_total = I_Na + I_K;
-    s.in[0] = (float)(((double)s.in[0]) - (I_Na * dt) / cpm);
-    s.in[1] = (float)(((double)s.in[1]) - (I_K * dt) / cpm);
+    s.in[0] = (float)(((double)s.in[0]) - s.over_cpm(I_Na * dt));
+    s.in[1] = (float)(((double)s.in[1]) - s.over_cpm(I_K * dt));
     if (P_Ca_ratio > 0.0f) {
         double I_Ca = P_Ca * dp_ghk_div_c(s.gc, V, ((double)s.in[2]), ((double)s.out[2])) * N * open_prob * mod_scale * A_TO_PA;
         I_total += I_Ca;
-        s.in[2] = (float)(((double)s.in[2]) - (I_Ca * dt) / (2.0f * cpm));
+        s.in[2] = (float)(((double)s.in[2]) - 0.5 * s.over_cpm(I_Ca * dt));
     }
     dp_clamp_ions(s.in);
     return -I_total;
