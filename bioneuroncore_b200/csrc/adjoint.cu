@@ -29,10 +29,20 @@
 //   intracellular Nernst-Planck sub-steps (hand-derived: Bernoulli fluxes, chord
 //   conductances, the transposed Jacobi sweeps) -> the phi_e solve -> step 1 (local
 //   Jacobians of the channel models by dual numbers, slot order reversed).
+//
+// What bounds it: instruction issue behind latency (forward 43% of issue slots at 14 warps
+// per SM, backward 30% at 8, its 230 registers the limit).  64 neurons x 64 segments, 16
+// sets, 160 ticks: forward 42.2 -> 11.0 ms, backward 139.7 -> 67.0, by what the plain tick
+// does too (one Bernoulli pair per valence, corrected quotients, a phi_e solve left at its
+// fixed point), the channel models in line, their items and each synapse's place in the
+// release log in shared memory, two-entry sweeps, and twice the forward CTAs per SM.
 #define BNC_MATH_OUTLINE 1   // one copy of exp/log for the forward, the re-runs and the reverse
 #ifndef BNC_ADJ_MIN_BLOCKS
 #define BNC_ADJ_MIN_BLOCKS 4   // CTAs per SM the 64-thread backward is bounded for (5 spills: slower)
 #endif
+#ifndef BNC_ADJ_FWD_BLOCKS
+#define BNC_ADJ_FWD_BLOCKS 8   // and the 64-thread forward and re-run: 128 registers (8: 15.3 ms, 7: 15.1, 10: 18.5,
+#endif                         // 6: 21.1, unbounded at 230 registers: 19.0; 64 neurons x 64, 16 sets, 160 ticks)
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -138,13 +148,18 @@ struct Lay {
     double *ibuf, *phiA, *phiB, *sig, *diag, *god, *ib3, *fa, *fb;
     unsigned long long* pmask;   // reverse pass: per segment, the phi_e sweeps that did not clamp
     float *st, *gax, *term, *vnA, *vnB;
+    float* coef;        // [7][Emax] D area dt_sub / length, fixed for the run
+    int* nphi;          // sweeps the phi_e solve ran before its iterate stopped changing
+    uint32_t* itw;      // [items][S] an item's type | its first gate word << 8 | default parameters << 16
+    float* iden;        // [items][S] its density
+    uint32_t* evc;      // [Y] each synapse's first release at or after the last tick run
     // reverse pass only
     float *s2, *lam, *lphi, *lI, *mu, *lvB, *linp, *lgdg, *eca, *ecb, *edv, *ldiag, *jsm;
 };
 
 __host__ __device__ inline size_t lay_bytes(uint32_t S, uint32_t E, uint32_t Y, bool bwd, uint32_t W) {
     size_t dbl = (size_t)6 * S + 15 * (size_t)E;
-    size_t flt = (size_t)W * S + kSynWords * Y + 2 * (size_t)E + 2 * (size_t)S;
+    size_t flt = (size_t)W * S + kSynWords * Y + 2 * (size_t)E + 2 * (size_t)S + 7 * (size_t)E + 1 + 2 * kItems * (size_t)S + Y;
     if (bwd) {
         dbl += S;   // pmask
         flt += 15 * (size_t)S + W * (size_t)S + kSynWords * (size_t)Y + 7 * (size_t)S + (size_t)E + 51 * (size_t)S + 4;
@@ -163,6 +178,11 @@ __device__ inline Lay make_lay(unsigned char* base, uint32_t S, uint32_t E, uint
     l.st = f; f += W * S + kSynWords * Y;
     l.gax = f; f += E; l.term = f; f += E;
     l.vnA = f; f += S; l.vnB = f; f += S;
+    l.coef = f; f += 7 * E;
+    l.nphi = reinterpret_cast<int*>(f); f += 1;
+    l.itw = reinterpret_cast<uint32_t*>(f); f += kItems * S;
+    l.iden = f; f += kItems * S;
+    l.evc = reinterpret_cast<uint32_t*>(f); f += Y;
     if (bwd) {
         l.s2 = f; f += 15 * S;
         l.lam = f; f += W * S + kSynWords * Y;   // the state's layout: segment words, then synapse words
@@ -189,7 +209,7 @@ struct Ctx {
     uint32_t L_n;          // block length
     // segment threadIdx.x (when < S): incident connections in original order, packed
     // as local id | other endpoint << 8 | (this is endpoint a) << 16 | intracellular << 17
-    uint32_t g, ninc;
+    uint32_t g, ninc, nit;
     uint32_t inc[kMaxInc];
     float cm, area;
     double vol;
@@ -197,6 +217,8 @@ struct Ctx {
     uint32_t ea, eb;
     bool eintra;
     float earea, edist, eva, evb;
+    double yva, yvb;       // 1 / eva, 1 / evb
+    bool two;              // no segment of the neuron has more than two connections
 };
 
 __device__ inline Ctx make_ctx(const AdjDev& d) {
@@ -211,13 +233,14 @@ __device__ inline Ctx make_ctx(const AdjDev& d) {
     c.L_n = d.nr_st[c.n + 1] - d.nr_st[c.n];
     const uint32_t tid = threadIdx.x;
     c.g = c.s0 + (tid < c.S ? tid : 0);
-    c.ninc = 0;
+    c.ninc = c.nit = 0;
 #pragma unroll
     for (int k = 0; k < kMaxInc; k++) c.inc[k] = 0;
     c.cm = c.area = 0.0f;
     c.vol = 0.0;
     if (tid < c.S) {
         c.ninc = d.inc_n[c.g];
+        c.nit = d.n_it[c.g];
         c.cm = d.cm[c.g];
         c.area = d.area[c.g];
         c.vol = d.vol[c.g];
@@ -234,12 +257,15 @@ __device__ inline Ctx make_ctx(const AdjDev& d) {
     c.ea = c.eb = 0;
     c.eintra = false;
     c.earea = c.edist = c.eva = c.evb = 1.0f;
+    c.yva = c.yvb = 1.0;
+    c.two = __syncthreads_and(c.ninc <= 2) != 0;
     if (tid < c.E) {
         const uint32_t e = c.e0 + tid;
         c.ea = d.ed_a[e]; c.eb = d.ed_b[e];
         c.eintra = d.ed_intra[e] != 0;
         c.earea = d.ed_area[e]; c.edist = d.ed_dist[e];
         c.eva = d.ed_vola[e]; c.evb = d.ed_volb[e];
+        c.yva = 1.0 / (double)c.eva; c.yvb = 1.0 / (double)c.evb;
     }
     return c;
 }
@@ -265,11 +291,45 @@ __device__ inline void block_store(float* dst, const float* src, const Ctx& c, u
     }
 }
 
+// The connections' Nernst-Planck coefficients, the same in every sub-step of the run.
+__device__ inline void coef_fill(const AdjDev& d, const Ctx& c, const Lay& L) {
+    const float dt_sub = d.dt / 5;
+    if (threadIdx.x < c.E)
+        for (int q = 0; q < 7; q++) L.coef[q * d.Emax + threadIdx.x] = c_D[q] * c.earea * dt_sub / c.edist;
+}
+
 __device__ inline float bern_f(float x) {
     if (fabsf(x) < 1e-3f) return 1.0f - 0.5f * x;
     if (x > 50.0f) return 0.0f;
     if (x < -50.0f) return -x;
     return x / (dm_exp(x) - 1.0f);
+}
+
+// bern_f at -x and x for valences +1 (0), +2 (1) and -1 (2, the first pair exchanged: its
+// argument is minus x), the two exponentials of a pair side by side.
+__device__ inline void bern_pairs(float x1, float (&bm)[3], float (&bp)[3]) {
+#pragma unroll
+    for (int g = 0; g < 2; g++) {
+        const float x = g ? 2.0f * x1 : x1;
+        const float ax = fabsf(x);
+        if (ax < 50.0f) {
+            const float lm = 1.0f - 0.5f * -x, lp = 1.0f - 0.5f * x;
+            bm[g] = lm;
+            bp[g] = lp;
+            if (ax >= 1e-3f) {
+                double em, ep;
+                if (ax < 0.34f) { em = dm_exp_taylor((double)-x); ep = dm_exp_taylor((double)x); }
+                else { em = dm_exp_mid((double)-x); ep = dm_exp_mid((double)x); }
+                bm[g] = (float)((double)-x / (em - 1.0));
+                bp[g] = (float)((double)x / (ep - 1.0));
+            }
+        } else {
+            bm[g] = bern_f(-x);
+            bp[g] = bern_f(x);
+        }
+    }
+    bm[2] = bp[0];
+    bp[2] = bm[0];
 }
 
 __device__ inline float par_of(const AdjDev& d, uint32_t p, int cls, uint32_t g) {
@@ -295,21 +355,42 @@ __device__ inline float den_of(const AdjDev& d, uint32_t p, uint8_t type, uint32
     return cls >= 0 ? par_of(d, p, cls, g) : d.it_den[g * kItems + j];
 }
 
-// the logged cleft entries of `slot` at `tick` (sorted by tick, then the order the
-// tick added them)
-__device__ inline float cleft_events(const AdjDev& d, uint32_t slot, unsigned long long tick, float cleft) {
-    uint32_t lo = d.ev_off[slot], hi = d.ev_off[slot + 1];
-    const uint32_t end = hi;
-    while (lo < hi) {
-        const uint32_t mid = (lo + hi) >> 1;
-        if (d.ev_tick[mid] < tick) lo = mid + 1; else hi = mid;
-    }
-    for (uint32_t q = lo; q < end && d.ev_tick[q] == tick; q++) cleft += d.ev_amt[q];
+// The logged cleft entries of `slot` at `tick` (sorted by tick, then the order the tick
+// added them).  cur: the slot's place in the log, which moves with the ticks either way.
+__device__ inline float cleft_events(const AdjDev& d, uint32_t slot, unsigned long long tick, float cleft, uint32_t& cur) {
+    const uint32_t beg = d.ev_off[slot], end = d.ev_off[slot + 1];
+    uint32_t q = min(max(cur, beg), end);
+    while (q < end && d.ev_tick[q] < tick) q++;
+    while (q > beg && d.ev_tick[q - 1] >= tick) q--;
+    cur = q;
+    for (; q < end && d.ev_tick[q] == tick; q++) cleft += d.ev_amt[q];
     return cleft;
 }
 
-// One differentiable item (kernel_dispatch.h:337-570 for its type), out of line so the
-// forward tick and the reverse tick's re-run share one copy of each model.
+// What a launch's ticks read of the neuron's items and release log, into shared memory.
+template <bool kFull>
+__device__ inline void items_fill(const AdjDev& d, const Ctx& c, const Lay& L) {
+    constexpr uint32_t IS = ItemStride<kFull>::v;
+    if (threadIdx.x < c.S) {
+        const uint32_t ni = d.n_it[c.g];
+        for (uint32_t j = 0; j < ni; j++) {
+            const uint8_t type = d.it_type[c.g * IS + j];
+            const float* st = d.it_st + ((size_t)c.g * IS + j) * 7;
+            // the parameter words of the types (zero: the default); the pump has none
+            bool def = true;
+            if (type == 141 || type == 142) def = st[5] == 0.0f;
+            else if (type == 123) def = st[1] == 0.0f && st[2] == 0.0f && st[4] == 0.0f;
+            else if (type == 107) def = st[0] == 0.0f && st[1] == 0.0f;
+            else if (type == 1) def = st[2] == 0.0f && st[3] == 0.0f && st[4] == 0.0f;
+            L.itw[j * d.Smax + threadIdx.x] = type | (uint32_t)d.it_gate[c.g * IS + j] << 8 | (def ? 1u << 16 : 0u);
+            L.iden[j * d.Smax + threadIdx.x] = kFull ? den_of(d, c.p, type, c.g, j) : par_of(d, c.p, cls_k<kFull>(type), c.g);
+        }
+    }
+    for (uint32_t y = threadIdx.x; y < c.Y; y += blockDim.x) L.evc[y] = d.ev_off[c.y0 + y];
+}
+
+// One differentiable item (kernel_dispatch.h:337-570 for its type) with parameters of its
+// own; the default ones run in line.
 __device__ __noinline__ double run_slot(uint8_t type, DMod& m, DSeg& s, float dt) {
     if (type == 123) return dp_kvdr_current<false>(m, s, dt);
     if (type == 107) return dp_k2p_current<false>(m, s, dt);
@@ -337,17 +418,25 @@ __device__ inline double step1_seg(const AdjDev& d, const Ctx& c, const Lay& L, 
     s.area = c.area;
     s.vol = c.vol;
     dp_seg_derived(s);
-    ghk_cache_fill(s.gc, s.V);
+    ghk_mono_fill(s.gc, s.V);
     double I_total = 0.0;
-    const uint32_t ni = d.n_it[g];
+    const uint32_t ni = c.nit;
+#pragma unroll 1
     for (uint32_t j = 0; j < ni; j++) {
         constexpr uint32_t IS = ItemStride<kFull>::v;
-        const uint8_t type = d.it_type[g * IS + j];
-        const uint32_t go = d.it_gate[g * IS + j];
+        const uint32_t itw = L.itw[j * Sm + i];
+        const uint8_t type = (uint8_t)(itw & 0xFFu);
+        const uint32_t go = (itw >> 8) & 0xFFu;
+        const bool def = (itw >> 16) != 0u;
+        if (__float_as_uint(s.V) != __float_as_uint(s.gc.Vc)) ghk_mono_fill(s.gc, s.V);
         DMod m;
-        m.den = kFull ? den_of(d, c.p, type, g, j) : par_of(d, c.p, cls_k<kFull>(type), g);
+        m.den = L.iden[j * Sm + i];
 #pragma unroll
-        for (int k = 0; k < 7; k++) m.st[k] = d.it_st[((size_t)g * IS + j) * 7 + k];
+        for (int k = 0; k < 7; k++) m.st[k] = 0.0f;
+        if (!def) {
+#pragma unroll
+            for (int k = 0; k < 7; k++) m.st[k] = d.it_st[((size_t)g * IS + j) * 7 + k];
+        }
         m.area = s.area;
         m.av = 0;
         const int ng = gates_k<kFull>(type);
@@ -368,7 +457,14 @@ __device__ inline double step1_seg(const AdjDev& d, const Ctx& c, const Lay& L, 
                 pre[(j * 5 + 4) * Sm + i] = ca ? s.out[2] : (na ? s.out[0] : s.out[1]);
             }
         }
-        I_total += run_slot(type, m, s, dt);
+        double I;
+        if (!def) { if (kFull) ghk_div_fill(s.gc, s.V); I = run_slot(type, m, s, dt); }
+        else if (type == 123) I = dp_kvdr_current<true>(m, s, dt);
+        else if (type == 107) I = dp_k2p_current<true>(m, s, dt);
+        else if (kFull && type == 1) { ghk_div_fill(s.gc, s.V); I = dp_cav13_current<true>(m, s, dt); }
+        else if (kFull && type == 7) I = dp_nak_pump_current(m, s, dt);
+        else I = dp_nav_current<true>(m, s, dt, type == 142 ? 1 : 0);
+        I_total += I;
         if (ng > 0) st[(15 + go) * Sm + i] = m.st[0];
         if (ng > 1) st[(16 + go) * Sm + i] = m.st[1];
     }
@@ -455,35 +551,55 @@ __device__ __forceinline__ void tick_fwd(const AdjDev& d, const Ctx& c, const La
             L.diag[tid] = diag;
             ib = L.ibuf[tid];
         }
+        // The stencil in registers; the diagonal's quotient as a corrected product.  A sweep
+        // maps an iterate to the next, so when one returns its iterate unchanged in every
+        // bit (after about 9) the rest of the 50 would too, and the solve stops; the
+        // reverse pass takes the sweeps not run from the last one.
         double* ph = L.phiA;
         double* pn = L.phiB;
+        double gg[kMaxInc];
+        uint32_t go[kMaxInc];
+#pragma unroll
+        for (int k = 0; k < kMaxInc; k++) {
+            gg[k] = ((uint32_t)k < c.ninc) ? L.god[inc_le(c.inc[k])] : 0.0;
+            go[k] = inc_o(c.inc[k]);
+        }
+        const bool live = diag > 1e-9;
+        const double ydiag = live ? 1.0 / diag : 1.0;
         unsigned long long unclamped = 0ull;
+        int nphi = 0;
         for (int it = 0; it < 50; it++) {
+            bool same = true;
             if (seg) {
-                if (kRec) sc.phs[it * Sm + tid] = (float)ph[tid];
+                const double old = ph[tid];
+                if (kRec) sc.phs[it * Sm + tid] = (float)old;
                 double acc = 0.0;
 #pragma unroll
-                for (int k = 0; k < kMaxInc; k++) {
-                    if ((uint32_t)k >= c.ninc) break;
-                    const double gg = L.god[inc_le(c.inc[k])];
-                    if (gg <= 0.0) continue;
-                    acc += gg * ph[inc_o(c.inc[k])];
-                }
-                double v = (diag > 1e-9) ? (acc - ib) / diag : 0.0;
-                if (kRec && diag > 1e-9 && v >= -10.0 && v <= 10.0) unclamped |= 1ull << it;
+                for (int k = 0; k < kMaxInc; k++)
+                    if (gg[k] > 0.0) acc += gg[k] * ph[go[k]];
+                double v = live ? dp_div_y(acc - ib, diag, ydiag) : 0.0;
+                if (kRec && live && v >= -10.0 && v <= 10.0) unclamped |= 1ull << it;
                 if (v > 10.0) v = 10.0;
                 if (v < -10.0) v = -10.0;
                 pn[tid] = v;
+                same = __double_as_longlong(v) == __double_as_longlong(old);
             }
-            __syncthreads();
+            nphi = it + 1;
+            const bool done = __syncthreads_and(same) != 0;
             double* tmp = ph; ph = pn; pn = tmp;
+            if (done) break;
         }
-        // 50 sweeps: the final phi is in phiA
+        // phiA and phiB hold the same values at a fixed point; 50 sweeps end in phiA
         const double* phi = ph;
-        if (kRec && seg) L.pmask[tid] = unclamped;
+        if (kRec && seg) {
+            if ((unclamped >> (nphi - 1)) & 1ull) unclamped |= ~0ull << (nphi - 1);
+            L.pmask[tid] = unclamped;
+            if (tid == 0) *L.nphi = nphi;
+        }
 
         // intracellular Nernst-Planck, 5 sub-steps (diffusion_kernel.h:152-238)
         float C_dt = 1.0f;
+        const double ydts = 1.0 / (double)dt_sub;
         if (seg) {
             C_dt = c.cm / dt_sub;
             if (C_dt < 1e-9f) C_dt = 1e-9f;
@@ -496,20 +612,26 @@ __device__ __forceinline__ void tick_fwd(const AdjDev& d, const Ctx& c, const La
             if (edge && c.eintra) {
                 const uint32_t a = c.ea, b = c.eb;
                 float sigma_i = 0.0f;
-                for (int q = 0; q < 7; q++) {
-                    float C_bar = (float)(0.5f * ((double)st[(1 + q) * Sm + a] + (double)st[(1 + q) * Sm + b]));
+                for (int q = 0; q < 7; q++) {   // the float mean is the binary64 one rounded
+                    const float C_bar = 0.5f * (st[(1 + q) * Sm + a] + st[(1 + q) * Sm + b]);
                     sigma_i += c_z2d[q] * C_bar;
                 }
                 const float g_ax = 3.612f * sigma_i * c.earea / c.edist;
                 const float dV = (float)(((double)st[a] + phi[a]) - ((double)st[b] + phi[b]));
+                // ions of equal valence share their Bernoulli values; the argument for
+                // z = -1 is minus the one for z = +1
+                float bm[3], bp[3];
+                bern_pairs(0.03742f * dV, bm, bp);
                 float I_np = 0.0f;
+#pragma unroll
                 for (int q = 0; q < 7; q++) {
+                    const int g = (q == 2 || q == 4) ? 1 : ((q == 3 || q == 5) ? 2 : 0);
                     const float C_a = st[(1 + q) * Sm + a], C_b = st[(1 + q) * Sm + b];
-                    const float x = c_z[q] * 0.03742f * dV;
-                    const float flux = c_D[q] * c.earea * dt_sub / c.edist * (C_a * bern_f(-x) - C_b * bern_f(x));
-                    L.fa[q * Em + tid] = (double)flux / c.eva;
-                    L.fb[q * Em + tid] = (double)flux / c.evb;
-                    I_np += c_z[q] * 96.485f * flux / dt_sub;
+                    const float flux = L.coef[q * Em + tid] * (C_a * bm[g] - C_b * bp[g]);
+                    L.fa[q * Em + tid] = dp_div_y((double)flux, (double)c.eva, c.yva);
+                    L.fb[q * Em + tid] = dp_div_y((double)flux, (double)c.evb, c.yvb);
+                    // the float quotient is the binary64 one rounded again
+                    I_np += (float)dp_div_y((double)(c_z[q] * 96.485f * flux), (double)dt_sub, ydts);
                 }
                 L.gax[tid] = g_ax;
                 L.term[tid] = I_np - g_ax * dV;
@@ -537,25 +659,87 @@ __device__ __forceinline__ void tick_fwd(const AdjDev& d, const Ctx& c, const La
                 vold = st[tid];
                 L.vnA[tid] = vold;
             }
-            __syncthreads();
             float* vn = L.vnA;
             float* vx = L.vnB;
             const float den = C_dt + gd;
-            for (int it = 0; it < 50; it++) {
-                if (seg) {
-                    if (kRec) sc.jac[(sub * 51 + it) * Sm + tid] = vn[tid];
-                    float offd = 0.0f;
+            const float rhs = C_dt * vold + ip;
+            float gx[kMaxInc];
+            uint32_t gxo[kMaxInc];
+            bool pos = true;
 #pragma unroll
-                    for (int k = 0; k < kMaxInc; k++) {
-                        if ((uint32_t)k >= c.ninc) break;
-                        const uint32_t w = c.inc[k];
-                        if (!inc_intra(w)) continue;
-                        offd += L.gax[inc_le(w)] * vn[inc_o(w)];
+            for (int k = 0; k < kMaxInc; k++) {
+                const uint32_t w = c.inc[k];
+                const bool on = (uint32_t)k < c.ninc && inc_intra(w);
+                gx[k] = on ? L.gax[inc_le(w)] : 0.0f;
+                gxo[k] = on ? inc_o(w) : 0u;
+                pos &= gx[k] >= 0.0f;
+            }
+            // Conditions under which every quotient of the solve is the IEEE one by a
+            // corrected product (the iterates stay within the largest |V_m| and
+            // |rhs| / C_dt, and rhs + off is 0 or above 2^-85): checked once per solve.
+            const float yden = 1.0f / den;
+            const bool ok = !seg || (pos && den >= 0x1p-32f && den <= 0x1p32f && fabsf(vold) <= 0x1p60f &&
+                                     fabsf(rhs) <= 0x1p60f && fabsf(rhs) >= 0x1p-60f);
+            const bool fast = __syncthreads_and(ok) != 0;
+            if (fast && c.two) {
+                // two stencil entries, two sweeps per turn (a missing one is 0 x this value)
+                const float g0 = gx[0], g1 = gx[1];
+                const uint32_t own = seg ? tid : 0u;
+                const float *a0 = L.vnA + (g0 != 0.0f ? gxo[0] : own), *a1 = L.vnA + (g1 != 0.0f ? gxo[1] : own);
+                const ptrdiff_t ab = L.vnB - L.vnA;
+                float* rec = sc.jac + (size_t)(sub * 51) * Sm + tid;
+                float v = vold;
+#pragma unroll 5
+                for (int it = 0; it < 50; it += 2) {
+                    if (seg) {
+                        if (kRec) { *rec = v; rec += Sm; }
+                        const float a = rhs + (g0 * a0[0] + g1 * a1[0]);
+                        const float q0 = a * yden;
+                        v = __fmaf_rn(__fmaf_rn(-q0, den, a), yden, q0);
+                        L.vnB[tid] = v;
                     }
-                    vx[tid] = (C_dt * vold + ip + offd) / den;
+                    __syncthreads();
+                    if (seg) {
+                        if (kRec) { *rec = v; rec += Sm; }
+                        const float a = rhs + (g0 * a0[ab] + g1 * a1[ab]);
+                        const float q0 = a * yden;
+                        v = __fmaf_rn(__fmaf_rn(-q0, den, a), yden, q0);
+                        L.vnA[tid] = v;
+                    }
+                    __syncthreads();
                 }
-                __syncthreads();
-                float* tmp = vn; vn = vx; vx = tmp;
+            } else if (fast) {
+                for (int it = 0; it < 50; it++) {
+                    if (seg) {
+                        if (kRec) sc.jac[(sub * 51 + it) * Sm + tid] = vn[tid];
+                        float offd = 0.0f;
+#pragma unroll
+                        for (int k = 0; k < kMaxInc; k++)
+                            if ((uint32_t)k < c.ninc) offd += gx[k] * vn[gxo[k]];
+                        const float a = rhs + offd;
+                        const float q0 = a * yden;
+                        vx[tid] = __fmaf_rn(__fmaf_rn(-q0, den, a), yden, q0);
+                    }
+                    __syncthreads();
+                    float* tmp = vn; vn = vx; vx = tmp;
+                }
+            } else {
+                for (int it = 0; it < 50; it++) {
+                    if (seg) {
+                        if (kRec) sc.jac[(sub * 51 + it) * Sm + tid] = vn[tid];
+                        float offd = 0.0f;
+#pragma unroll
+                        for (int k = 0; k < kMaxInc; k++) {
+                            if ((uint32_t)k >= c.ninc) break;
+                            const uint32_t w = c.inc[k];
+                            if (!inc_intra(w)) continue;
+                            offd += L.gax[inc_le(w)] * vn[inc_o(w)];
+                        }
+                        vx[tid] = (rhs + offd) / den;
+                    }
+                    __syncthreads();
+                    float* tmp = vn; vn = vx; vx = tmp;
+                }
             }
             if (seg) {
                 if (kRec) sc.jac[(sub * 51 + 50) * Sm + tid] = vn[tid];
@@ -568,25 +752,23 @@ __device__ __forceinline__ void tick_fwd(const AdjDev& d, const Ctx& c, const La
 
         // extracellular Nernst-Planck, 5 sub-steps (diffusion_kernel.h:244-281); the
         // Bernoulli factors depend on phi_e only
-        float bm[7], bp[7];
+        float bm[3], bp[3];
         if (edge) {
             const double dphi = phi[c.ea] - phi[c.eb];
-            for (int q = 0; q < 7; q++) {
-                const float x = (float)(c_z[q] * 0.03742f * dphi);
-                bm[q] = bern_f(-x);
-                bp[q] = bern_f(x);
-            }
+            bern_pairs((float)(0.03742f * dphi), bm, bp);
         }
-        const float vea = c.eva * EXTRA_VOLUME_RATIO, veb = c.evb * EXTRA_VOLUME_RATIO;
+        // the extracellular volumes are 0.25 x the intracellular ones
         for (int sub = 0; sub < 5; sub++) {
             if (kRec && seg)
                 for (int q = 0; q < 7; q++) sc.estart[(sub * 7 + q) * Sm + tid] = st[(8 + q) * Sm + tid];
             if (edge) {
+#pragma unroll
                 for (int q = 0; q < 7; q++) {
+                    const int g = (q == 2 || q == 4) ? 1 : ((q == 3 || q == 5) ? 2 : 0);
                     const double Ca = st[(8 + q) * Sm + c.ea], Cb = st[(8 + q) * Sm + c.eb];
-                    const double flux = c_D[q] * c.earea * dt_sub / c.edist * (Ca * bm[q] - Cb * bp[q]);
-                    L.fa[q * Em + tid] = flux / vea;
-                    L.fb[q * Em + tid] = flux / veb;
+                    const double flux = L.coef[q * Em + tid] * (Ca * bm[g] - Cb * bp[g]);
+                    L.fa[q * Em + tid] = 4.0 * dp_div_y(flux, (double)c.eva, c.yva);
+                    L.fb[q * Em + tid] = 4.0 * dp_div_y(flux, (double)c.evb, c.yvb);
                 }
             }
             __syncthreads();
@@ -672,7 +854,7 @@ __device__ __forceinline__ void tick_fwd(const AdjDev& d, const Ctx& c, const La
         float* rs = st + (kFull ? d.W : kW3) * Sm;
         for (uint32_t y = d.sp_off[g]; y < d.sp_off[g + 1]; y++) {
             const uint32_t ly = y - c.y0;
-            float cleft = cleft_events(d, y, tick, rs[ly * kSynWords + 4]);
+            float cleft = cleft_events(d, y, tick, rs[ly * kSynWords + 4], L.evc[ly]);
             if (d.sl_nt[y] == 0) nt_glu += cleft;
             else if (d.sl_nt[y] == 1) nt_gaba += cleft;
             else nt_gly += cleft;
@@ -882,26 +1064,29 @@ __device__ void tick_rev(const AdjDev& d, const Ctx& c, const Lay& L, const Scr&
         }
         // ---- extracellular sub-steps, last first ----
         float elphi = 0.0f;
-        float bm[7], bp[7], dbm[7], dbp[7], kq[7];
+        float bm[3], bp[3], dbm[3], dbp[3];   // per valence +1, +2, -1
         if (edge) {
             const double dphi = phiF[c.ea] - phiF[c.eb];
-            for (int q = 0; q < 7; q++) {
-                const float x = (float)(c_z[q] * 0.03742f * dphi);
-                adj::bern_pair(x, dm_expf(x), &bp[q], &dbp[q]);
-                bm[q] = bp[q] + x;
-                dbm[q] = -(dbp[q] + 1.0f);
-                kq[q] = c_D[q] * c.earea * dt_sub / c.edist;
+#pragma unroll
+            for (int g = 0; g < 3; g++) {
+                const float x = (float)((g == 0 ? 1.0f : g == 1 ? 2.0f : -1.0f) * 0.03742f * dphi);
+                adj::bern_pair(x, dm_expf(x), &bp[g], &dbp[g]);
+                bm[g] = bp[g] + x;
+                dbm[g] = -(dbp[g] + 1.0f);
             }
         }
         const float rvea = 1.0f / (c.eva * EXTRA_VOLUME_RATIO), rveb = 1.0f / (c.evb * EXTRA_VOLUME_RATIO);
         for (int sub = 4; sub >= 0; sub--) {
             if (edge) {
+#pragma unroll
                 for (int q = 0; q < 7; q++) {
+                    const int g = (q == 2 || q == 4) ? 1 : ((q == 3 || q == 5) ? 2 : 0);
+                    const float kq = L.coef[q * Em + tid];
                     const float Ca = sc.estart[(sub * 7 + q) * Sm + c.ea], Cb = sc.estart[(sub * 7 + q) * Sm + c.eb];
                     const float lf = -lam[(8 + q) * Sm + c.ea] * rvea + lam[(8 + q) * Sm + c.eb] * rveb;
-                    L.eca[q * Em + tid] = lf * kq[q] * bm[q];
-                    L.ecb[q * Em + tid] = -lf * kq[q] * bp[q];
-                    elphi += lf * kq[q] * (-Ca * dbm[q] - Cb * dbp[q]) * (c_z[q] * 0.03742f);
+                    L.eca[q * Em + tid] = lf * kq * bm[g];
+                    L.ecb[q * Em + tid] = -lf * kq * bp[g];
+                    elphi += lf * kq * (-Ca * dbm[g] - Cb * dbp[g]) * (c_z[q] * 0.03742f);
                 }
             }
             __syncthreads();
@@ -944,23 +1129,22 @@ __device__ void tick_rev(const AdjDev& d, const Ctx& c, const Lay& L, const Scr&
             float gax = 0.0f, dVe = 0.0f;
             if (edge && c.eintra) {
                 float sigma_i = 0.0f;
-                for (int q = 0; q < 7; q++) {
-                    float C_bar = (float)(0.5f * ((double)Is[q * Sm + c.ea] + (double)Is[q * Sm + c.eb]));
-                    sigma_i += c_z2d[q] * C_bar;
-                }
+                for (int q = 0; q < 7; q++) sigma_i += c_z2d[q] * (0.5f * (Is[q * Sm + c.ea] + Is[q * Sm + c.eb]));
                 gax = 3.612f * sigma_i * c.earea / c.edist;
                 dVe = (float)(((double)Vs[c.ea] + phiF[c.ea]) - ((double)Vs[c.eb] + phiF[c.eb]));
             }
             if (edge) L.gax[tid] = gax;
             __syncthreads();
             float gdiag = 0.0f, lVold = 0.0f, linp = 0.0f, lgdg = 0.0f;
-            if (seg) {
+            float gx[kMaxInc];   // the sweeps' stencil
+            uint32_t gxo[kMaxInc];
 #pragma unroll
-                for (int k = 0; k < kMaxInc; k++) {
-                    if ((uint32_t)k >= c.ninc) break;
-                    const uint32_t w = c.inc[k];
-                    if (inc_intra(w)) gdiag += L.gax[inc_le(w)];
-                }
+            for (int k = 0; k < kMaxInc; k++) {
+                const uint32_t w = c.inc[k];
+                const bool on = (uint32_t)k < c.ninc && inc_intra(w);
+                gx[k] = on ? L.gax[inc_le(w)] : 0.0f;
+                gxo[k] = on ? inc_o(w) : 0u;
+                if (on) gdiag += gx[k];
             }
             const float rden = 1.0f / (C_dt + gdiag);
             // the sub-step's 51 iterates into shared memory: asynchronous 16-byte copies, all
@@ -978,6 +1162,33 @@ __device__ void tick_rev(const AdjDev& d, const Ctx& c, const Lay& L, const Scr&
             float lgo = 0.0f;
             float lv = seg ? lam[tid] : 0.0f;
             const float* js = L.jsm;
+            if (c.two) {   // two stencil entries, two sweeps per turn
+                const float g0 = gx[0], g1 = gx[1];
+                const uint32_t own = seg ? tid : 0u;
+                const uint32_t o0 = g0 != 0.0f ? gxo[0] : own, o1 = g1 != 0.0f ? gxo[1] : own;
+                const bool ed = edge && c.eintra;
+                const uint32_t ea = ed ? c.ea : 0u, eb = ed ? c.eb : 0u;
+                const float *ja = js + 49 * (size_t)Sm + ea, *jb = js + 49 * (size_t)Sm + eb;
+                const float* jt = js + 50 * (size_t)Sm + own;
+                auto turn = [&](float* mu) {
+                    if (seg) {
+                        const float m = lv * rden;
+                        lVold += C_dt * m;
+                        linp += m;
+                        lgdg -= m * *jt;
+                        mu[tid] = m;
+                    }
+                    __syncthreads();
+                    if (ed) lgo += mu[ea] * *jb + mu[eb] * *ja;
+                    if (seg) lv = g0 * mu[o0] + g1 * mu[o1];
+                    jt -= Sm; ja -= Sm; jb -= Sm;
+                };
+#pragma unroll 1
+                for (int k = 49; k >= 0; k -= 2) {
+                    turn(L.lvB);
+                    turn(L.mu);
+                }
+            } else
             for (int k = 49; k >= 0; k--) {
                 float* mu = (k & 1) ? L.lvB : L.mu;
                 if (seg) {
@@ -992,12 +1203,8 @@ __device__ void tick_rev(const AdjDev& d, const Ctx& c, const Lay& L, const Scr&
                 if (seg) {
                     float acc = 0.0f;
 #pragma unroll
-                    for (int q = 0; q < kMaxInc; q++) {
-                        if ((uint32_t)q >= c.ninc) break;
-                        const uint32_t w = c.inc[q];
-                        if (!inc_intra(w)) continue;
-                        acc += L.gax[inc_le(w)] * mu[inc_o(w)];
-                    }
+                    for (int q = 0; q < kMaxInc; q++)
+                        if ((uint32_t)q < c.ninc && inc_intra(c.inc[q])) acc += gx[q] * mu[gxo[q]];
                     lv = acc;
                 }
             }
@@ -1017,17 +1224,23 @@ __device__ void tick_rev(const AdjDev& d, const Ctx& c, const Lay& L, const Scr&
                     const float gfac = lgax * (3.612f * c.earea / c.edist) * 0.5f;
                     const float rva = 1.0f / c.eva, rvb = 1.0f / c.evb, kk = c.earea * dt_sub / c.edist;
                     const float inp_f = dl * 96.485f / dt_sub;
+                    float Bm[3], Bp[3], dBm[3], dBp[3];   // per valence +1, +2, -1
+#pragma unroll
+                    for (int g = 0; g < 3; g++) {
+                        const float x = (g == 0 ? 1.0f : g == 1 ? 2.0f : -1.0f) * 0.03742f * dVe;
+                        adj::bern_pair(x, dm_expf(x), &Bp[g], &dBp[g]);
+                        Bm[g] = Bp[g] + x;
+                        dBm[g] = -(dBp[g] + 1.0f);
+                    }
+#pragma unroll
                     for (int q = 0; q < 7; q++) {
+                        const int g = (q == 2 || q == 4) ? 1 : ((q == 3 || q == 5) ? 2 : 0);
                         const float Ca = Is[q * Sm + a], Cb = Is[q * Sm + b];
-                        const float x = c_z[q] * 0.03742f * dVe;
                         const float k = c_D[q] * kk;
                         const float lf = inp_f * c_z[q] - lam[(1 + q) * Sm + a] * rva + lam[(1 + q) * Sm + b] * rvb;
-                        float Bp, dBp;
-                        adj::bern_pair(x, dm_expf(x), &Bp, &dBp);
-                        const float Bm = Bp + x, dBm = -(dBp + 1.0f);
-                        L.eca[q * Em + tid] = lf * k * Bm + gfac * c_z2d[q];
-                        L.ecb[q * Em + tid] = -lf * k * Bp + gfac * c_z2d[q];
-                        ldV += lf * k * (-Ca * dBm - Cb * dBp) * (c_z[q] * 0.03742f);
+                        L.eca[q * Em + tid] = lf * k * Bm[g] + gfac * c_z2d[q];
+                        L.ecb[q * Em + tid] = -lf * k * Bp[g] + gfac * c_z2d[q];
+                        ldV += lf * k * (-Ca * dBm[g] - Cb * dBp[g]) * (c_z[q] * 0.03742f);
                     }
                     L.edv[tid] = ldV;
                 } else {
@@ -1068,46 +1281,47 @@ __device__ void tick_rev(const AdjDev& d, const Ctx& c, const Lay& L, const Scr&
         float lI = seg ? L.lI[tid] : 0.0f;
         float lg = 0.0f;
         const double god = edge ? L.god[tid] : 0.0;
-        const float godf = (float)god;
-        // the recorded iterates into shared memory (the Jacobi staging area is free here)
+        float gp[kMaxInc];
+#pragma unroll
+        for (int q = 0; q < kMaxInc; q++) gp[q] = (uint32_t)q < c.ninc ? (float)L.god[inc_le(c.inc[q])] : 0.0f;
+        // the recorded iterates into shared memory (the Jacobi staging area is free here);
+        // from the last sweep run on, they are that sweep's
+        const int nphi = *L.nphi;
         {
             const float4* src4 = reinterpret_cast<const float4*>(sc.phs);
             float4* dst4 = reinterpret_cast<float4*>(L.jsm);
-            for (uint32_t q = tid; q < 50u * Sm / 4u; q += blockDim.x) __pipeline_memcpy_async(dst4 + q, src4 + q, 16);
+            for (uint32_t q = tid; q < (uint32_t)nphi * Sm / 4u; q += blockDim.x) __pipeline_memcpy_async(dst4 + q, src4 + q, 16);
             __pipeline_commit();
             __pipeline_wait_prior(0);
         }
         __syncthreads();
         const float* phs = L.jsm;
+        const float unc49 = seg ? (float)L.phiA[tid] : 0.0f;
         for (int k = 49; k >= 0; k--) {
-            const float* ph = phs + (size_t)k * Sm;
+            const float* ph = phs + (size_t)min(k, nphi - 1) * Sm;
             float* mu = (k & 1) ? L.lvB : L.mu;
             if (seg) {
                 float m = 0.0f;
                 if ((pm >> k) & 1ull) {
                     m = lp * rdiag;
-                    const float unc = (k == 49) ? (float)L.phiA[tid] : phs[(k + 1) * Sm + tid];
+                    const float unc = (k == 49) ? unc49 : phs[(size_t)min(k + 1, nphi - 1) * Sm + tid];
                     ldg -= m * unc;
                 }
                 lI -= m;
                 mu[tid] = m;
             }
-            __syncthreads();
+            // the adjoint of the iterate shrinks by the diagonal's share each sweep and ends
+            // in zeros: nothing is left to add
+            if (!__syncthreads_or(seg && mu[tid] != 0.0f)) break;
             if (edge && god > 0.0) lg += mu[c.ea] * ph[c.eb] + mu[c.eb] * ph[c.ea];
             if (seg) {
                 float acc = 0.0f;
 #pragma unroll
-                for (int q = 0; q < kMaxInc; q++) {
-                    if ((uint32_t)q >= c.ninc) break;
-                    const uint32_t w = c.inc[q];
-                    const float gg = (float)L.god[inc_le(w)];
-                    if (gg <= 0.0f) continue;
-                    acc += gg * mu[inc_o(w)];
-                }
+                for (int q = 0; q < kMaxInc; q++)
+                    if (gp[q] > 0.0f) acc += gp[q] * mu[inc_o(c.inc[q])];
                 lp = acc;
             }
         }
-        (void)godf;
         __syncthreads();
         if (seg) { L.ldiag[tid] = ldg; L.lI[tid] = lI; }
         __syncthreads();
@@ -1133,16 +1347,22 @@ __device__ void tick_rev(const AdjDev& d, const Ctx& c, const Lay& L, const Scr&
     if (seg) {
         const uint32_t g = c.g;
         const float lIt = L.lI[tid];
-        const uint32_t ni = d.n_it[g];
+        const uint32_t ni = c.nit;
         float lV = lam[tid];
+        float nx[5];   // an item's recorded inputs, loaded one item ahead
+#pragma unroll
+        for (int k = 0; k < 5; k++) nx[k] = ni ? sc.pre[((ni - 1) * 5 + k) * Sm + tid] : 0.0f;
         for (int j = (int)ni - 1; j >= 0; j--) {
             constexpr uint32_t IS = ItemStride<kFull>::v;
-            const uint8_t type = d.it_type[g * IS + j];
-            const uint32_t go = d.it_gate[g * IS + j];
-            const float den = kFull ? den_of(d, c.p, type, g, j) : par_of(d, c.p, cls_k<kFull>(type), g);
-            const float pV = sc.pre[(j * 5 + 0) * Sm + tid], pG0 = sc.pre[(j * 5 + 1) * Sm + tid],
-                        pG1 = sc.pre[(j * 5 + 2) * Sm + tid], pCi = sc.pre[(j * 5 + 3) * Sm + tid],
-                        pCo = sc.pre[(j * 5 + 4) * Sm + tid];
+            const uint32_t itw = L.itw[j * Sm + tid];
+            const uint8_t type = (uint8_t)(itw & 0xFFu);
+            const uint32_t go = (itw >> 8) & 0xFFu;
+            const float den = L.iden[j * Sm + tid];
+            const float pV = nx[0], pG0 = nx[1], pG1 = nx[2], pCi = nx[3], pCo = nx[4];
+            if (j > 0) {
+#pragma unroll
+                for (int k = 0; k < 5; k++) nx[k] = sc.pre[((j - 1) * 5 + k) * Sm + tid];
+            }
             if (kFull && type == 7) {   // the pump: inputs V, Na_in, K_out, ATP (recorded in that order)
                 float lp[7] = {lV, lam[1 * Sm + tid], lam[8 * Sm + tid], lam[2 * Sm + tid], lam[9 * Sm + tid],
                                lam[d.atp_w * Sm + tid], lIt};
@@ -1192,13 +1412,15 @@ __global__ void k_adj_init(AdjDev d) {
 }
 
 // Forward pass over ticks [t0, t1): checkpoints every K ticks, the loss and the traces.
-template <bool kFull>
-__global__ void __launch_bounds__(kMaxSeg) k_adj_forward(AdjDev d, uint32_t t0, uint32_t t1) {
+template <bool kFull, int kThreads, int kMinBlocks>
+__global__ void __launch_bounds__(kThreads, kMinBlocks) k_adj_forward(AdjDev d, uint32_t t0, uint32_t t1) {
     extern __shared__ __align__(16) unsigned char smem[];
     const Ctx c = make_ctx(d);
     const Lay L = make_lay(smem, d.Smax, d.Emax, d.Ymax, false, d.W);
     const Scr sc{};
     float* gstate = d.state + (size_t)c.p * d.L + c.st_off;
+    coef_fill(d, c, L);
+    items_fill<kFull>(d, c, L);
     block_load(L.st, gstate, c, d.Smax, d.W);
     __syncthreads();
     double loss = 0.0;
@@ -1227,8 +1449,8 @@ __global__ void __launch_bounds__(kMaxSeg) k_adj_forward(AdjDev d, uint32_t t0, 
 // reverse launch: every CTA then runs the forward tick's code at the forward kernel's
 // occupancy, where in the reverse kernel CTAs re-running and CTAs reversing would share
 // an SM's instruction caches between the two ticks' code.
-template <bool kFull>
-__global__ void __launch_bounds__(kMaxSeg) k_adj_rerun(AdjDev d, uint32_t w) {
+template <bool kFull, int kThreads, int kMinBlocks>
+__global__ void __launch_bounds__(kThreads, kMinBlocks) k_adj_rerun(AdjDev d, uint32_t w) {
     extern __shared__ __align__(16) unsigned char smem[];
     const Ctx c = make_ctx(d);
     const uint32_t W = kFull ? d.W : kW3;
@@ -1236,6 +1458,8 @@ __global__ void __launch_bounds__(kMaxSeg) k_adj_rerun(AdjDev d, uint32_t w) {
     const Scr sc{};
     const uint32_t tb = w * d.K;
     const uint32_t te = min(d.T, tb + d.K);
+    coef_fill(d, c, L);
+    items_fill<kFull>(d, c, L);
     block_load(L.st, d.ckpt + ((size_t)w * d.n_sets + c.p) * d.L + c.st_off, c, d.Smax, W);
     __syncthreads();
     for (uint32_t t = tb; t < te; t++) {
@@ -1260,6 +1484,8 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) k_adj_backward(AdjDev d,
     const uint32_t tb = w * d.K;
     const uint32_t te = min(d.T, tb + d.K);
     const uint32_t Sm = d.Smax;
+    coef_fill(d, c, L);
+    items_fill<kFull>(d, c, L);
     {   // adjoint of the state at the window's end
         const float* src = d.lam + (size_t)c.p * d.L + c.st_off;
         block_load(L.lam, src, c, Sm, W);
@@ -1720,15 +1946,17 @@ int adj_build(Adjoint* A, void* sim, const BncAdjointConfig& cfg) {
     A->smem_fwd = lay_bytes(d.Smax, d.Emax, Ymax, false, Wseg);
     A->smem_bwd = lay_bytes(d.Smax, d.Emax, Ymax, true, Wseg);
     if (A->smem_bwd > 227u * 1024u) { set_error("adjoint: a neuron needs %zu bytes of shared memory", A->smem_bwd); return BNC_ERR_UNSUPPORTED; }
-    if (cudaFuncSetAttribute(k_adj_forward<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)A->smem_fwd) != cudaSuccess ||
-        cudaFuncSetAttribute(k_adj_forward<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)A->smem_fwd) != cudaSuccess ||
-        cudaFuncSetAttribute(k_adj_rerun<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)A->smem_fwd) != cudaSuccess ||
-        cudaFuncSetAttribute(k_adj_rerun<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)A->smem_fwd) != cudaSuccess ||
-        cudaFuncSetAttribute(k_adj_backward<false, kMaxSeg, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)A->smem_bwd) != cudaSuccess ||
-        cudaFuncSetAttribute(k_adj_backward<true, kMaxSeg, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)A->smem_bwd) != cudaSuccess ||
-        cudaFuncSetAttribute(k_adj_backward<false, 64, BNC_ADJ_MIN_BLOCKS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)A->smem_bwd) != cudaSuccess ||
-        cudaFuncSetAttribute(k_adj_backward<true, 64, BNC_ADJ_MIN_BLOCKS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)A->smem_bwd) != cudaSuccess)
-        return adj_fail(BNC_ERR_CUDA, "shared-memory limit");
+    // the limit is a property of the kernel, not of this object: the most any neuron needs
+    const void* kernels[] = {
+        (const void*)k_adj_forward<false, kMaxSeg, 1>, (const void*)k_adj_forward<true, kMaxSeg, 1>,
+        (const void*)k_adj_forward<false, 64, BNC_ADJ_FWD_BLOCKS>, (const void*)k_adj_forward<true, 64, BNC_ADJ_FWD_BLOCKS>,
+        (const void*)k_adj_rerun<false, kMaxSeg, 1>, (const void*)k_adj_rerun<true, kMaxSeg, 1>,
+        (const void*)k_adj_rerun<false, 64, BNC_ADJ_FWD_BLOCKS>, (const void*)k_adj_rerun<true, 64, BNC_ADJ_FWD_BLOCKS>,
+        (const void*)k_adj_backward<false, kMaxSeg, 1>, (const void*)k_adj_backward<true, kMaxSeg, 1>,
+        (const void*)k_adj_backward<false, 64, BNC_ADJ_MIN_BLOCKS>, (const void*)k_adj_backward<true, 64, BNC_ADJ_MIN_BLOCKS>};
+    for (const void* k : kernels)
+        if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024) != cudaSuccess)
+            return adj_fail(BNC_ERR_CUDA, "shared-memory limit");
     return BNC_OK;
 }
 
@@ -1913,8 +2141,13 @@ int bnc_adjoint_forward(void* adj, double* loss, float* trace) {
     const dim3 grid(d.nn, d.n_sets);
     for (uint32_t t0 = 0; t0 < d.T; t0 += d.K) {
         const uint32_t t1 = std::min(d.T, t0 + d.K);
-        if (d.full) k_adj_forward<true><<<grid, A->threads, A->smem_fwd, A->stream>>>(d, t0, t1);
-        else k_adj_forward<false><<<grid, A->threads, A->smem_fwd, A->stream>>>(d, t0, t1);
+        if (A->threads <= 64) {
+            if (d.full) k_adj_forward<true, 64, BNC_ADJ_FWD_BLOCKS><<<grid, A->threads, A->smem_fwd, A->stream>>>(d, t0, t1);
+            else k_adj_forward<false, 64, BNC_ADJ_FWD_BLOCKS><<<grid, A->threads, A->smem_fwd, A->stream>>>(d, t0, t1);
+        } else {
+            if (d.full) k_adj_forward<true, kMaxSeg, 1><<<grid, A->threads, A->smem_fwd, A->stream>>>(d, t0, t1);
+            else k_adj_forward<false, kMaxSeg, 1><<<grid, A->threads, A->smem_fwd, A->stream>>>(d, t0, t1);
+        }
     }
     cudaEventRecord(A->ev1, A->stream);
     cudaError_t e = cudaStreamSynchronize(A->stream);
@@ -1951,8 +2184,13 @@ int bnc_adjoint_backward(void* adj, float* g_gNa, float* g_gK, float* g_gleak, f
     cudaEventRecord(A->ev0, A->stream);
     const dim3 grid(d.nn, d.n_sets);
     for (int w = (int)d.n_ckpt - 1; w >= 0; w--) {
-        if (d.full) k_adj_rerun<true><<<grid, A->threads, A->smem_fwd, A->stream>>>(d, (uint32_t)w);
-        else k_adj_rerun<false><<<grid, A->threads, A->smem_fwd, A->stream>>>(d, (uint32_t)w);
+        if (A->threads <= 64) {
+            if (d.full) k_adj_rerun<true, 64, BNC_ADJ_FWD_BLOCKS><<<grid, A->threads, A->smem_fwd, A->stream>>>(d, (uint32_t)w);
+            else k_adj_rerun<false, 64, BNC_ADJ_FWD_BLOCKS><<<grid, A->threads, A->smem_fwd, A->stream>>>(d, (uint32_t)w);
+        } else {
+            if (d.full) k_adj_rerun<true, kMaxSeg, 1><<<grid, A->threads, A->smem_fwd, A->stream>>>(d, (uint32_t)w);
+            else k_adj_rerun<false, kMaxSeg, 1><<<grid, A->threads, A->smem_fwd, A->stream>>>(d, (uint32_t)w);
+        }
         if (A->threads <= 64) {
             if (d.full) k_adj_backward<true, 64, BNC_ADJ_MIN_BLOCKS><<<grid, A->threads, A->smem_bwd, A->stream>>>(d, (uint32_t)w);
             else k_adj_backward<false, 64, BNC_ADJ_MIN_BLOCKS><<<grid, A->threads, A->smem_bwd, A->stream>>>(d, (uint32_t)w);

@@ -276,11 +276,11 @@ __device__ __forceinline__ GhkD ghk_mono_d(double Vd, double ci, double co) {
     if (Vn > 20.0) { r.F = A * ci; r.dV = dA * ci; r.dci = A; r.dco = 0.0; return r; }
     if (Vn < -20.0) { r.F = A * co; r.dV = dA * co; r.dci = 0.0; r.dco = A; return r; }
     const double e = adj_exp(-Vn), de = -e * c1;
-    const double D = 1.0 - e, Nn = ci - co * e;
-    r.F = A * Nn / D;
-    r.dV = dA * Nn / D + A * de * (ci - co) / (D * D);
-    r.dci = A / D;
-    r.dco = -A * e / D;
+    const double R = 1.0 / (1.0 - e), Nn = ci - co * e;   // one division for the five quotients
+    r.dci = A * R;
+    r.F = r.dci * Nn;
+    r.dV = (dA * Nn + r.dci * de * (ci - co)) * R;
+    r.dco = -r.dci * e;
     return r;
 }
 
@@ -384,17 +384,17 @@ __device__ __forceinline__ void vjp_k2p(const double* lo, double* lx, float V0, 
 __device__ __forceinline__ void vjp_receptor(const double* lo, double* lx, int anion, double P_a, double P_b, float V0,
                                              const float* in, const float* out, float w, float den, float area,
                                              float open, double vol, float dt, float* nv) {
-    const double cpm = kF * vol / 1000.0;
+    const double T = (double)dt / (kF * vol / 1000.0);   // dt over the volume's charge per mole
     const double Nk = (double)den * (double)area * (double)open * 1e12;
     for (int k = 0; k < 8; k++) lx[k] = 0.0;
     nv[0] = in[0]; nv[1] = in[1]; nv[2] = in[3];
     if (anion) {
         const GhkD G = ghk_mono_d((double)V0, out[3], in[3]);   // anion flux: c_in and c_out swapped
         const double I = P_a * G.F * Nk * (double)w;
-        const double n3 = (double)in[3] + I * (double)dt / cpm;
+        const double n3 = (double)in[3] + I * T;
         const bool m3 = n3 >= 1e-9;
         nv[2] = (float)(m3 ? n3 : 1e-9);
-        const double lI = -lo[3] + (m3 ? lo[2] * (double)dt / cpm : 0.0);
+        const double lI = -lo[3] + (m3 ? lo[2] * T : 0.0);
         const double lF = lI * P_a * Nk * (double)w;
         lx[0] = lF * G.dV;
         lx[1] = lo[0]; lx[2] = lo[1];
@@ -406,12 +406,12 @@ __device__ __forceinline__ void vjp_receptor(const double* lo, double* lx, int a
     const GhkD Ga = ghk_mono_d((double)V0, in[0], out[0]);
     const GhkD Gb = ghk_mono_d((double)V0, in[1], out[1]);
     const double Ia = P_a * Ga.F * Nk * (double)w, Ib = P_b * Gb.F * Nk * (double)w;
-    const double n0 = (double)in[0] - Ia * (double)dt / cpm, n1 = (double)in[1] - Ib * (double)dt / cpm;
+    const double n0 = (double)in[0] - Ia * T, n1 = (double)in[1] - Ib * T;
     const bool m0 = n0 >= 1e-9, m1 = n1 >= 1e-9;
     nv[0] = (float)(m0 ? n0 : 1e-9);
     nv[1] = (float)(m1 ? n1 : 1e-9);
-    const double lIa = -lo[3] - (m0 ? lo[0] * (double)dt / cpm : 0.0);
-    const double lIb = -lo[3] - (m1 ? lo[1] * (double)dt / cpm : 0.0);
+    const double lIa = -lo[3] - (m0 ? lo[0] * T : 0.0);
+    const double lIb = -lo[3] - (m1 ? lo[1] * T : 0.0);
     const double lFa = lIa * P_a * Nk * (double)w, lFb = lIb * P_b * Nk * (double)w;
     lx[0] = lFa * Ga.dV + lFb * Gb.dV;
     lx[1] = (m0 ? lo[0] : 0.0) + lFa * Ga.dci;

@@ -367,10 +367,15 @@ __device__ __forceinline__ double dp_nav_current(DMod& m, DSeg& s, float dt, int
     if (((double)s.V) < -200.0f) s.V = -200.0f;
     if (((double)s.V) > 200.0f) s.V = 200.0f;
     V = (float)((double)s.V);
-    float minf = is12 ? nav12_m_inf(V) : nav16_m_inf(V);
-    float mtau = is12 ? nav12_m_tau(V) : nav16_m_tau(V);
-    float hinf = is12 ? nav12_h_inf(V) : nav16_h_inf(V);
-    float htau = is12 ? nav12_h_tau(V) : nav16_h_tau(V);
+    // the two channels' rates differ in their shifts only; each rate is formed once
+    const float am = 0.182f * dp_vtrap(V + (is12 ? 23.0f : 43.0f), 6.0f);
+    const float bm = 0.124f * dp_vtrap(-(V + (is12 ? 23.0f : 43.0f)), 6.0f);
+    const float ah = 0.024f * dp_vtrap(V + (is12 ? 41.5f : 50.0f), 5.0f);
+    const float bh = 0.0091f * dp_vtrap(-(V + (is12 ? 66.5f : 75.0f)), 5.0f);
+    float minf = am / (am + bm);
+    float mtau = 1.0f / (am + bm);
+    float hinf = 1.0f / (1.0f + dm_exp(fp_over(V + (is12 ? 63.5f : 72.0f), 6.2f)));
+    float htau = 1.0f / (ah + bh);
     double m_val = minf + (((double)m.st[0]) - minf) * dm_exp(-dt / mtau);
     double h_val = hinf + (((double)m.st[1]) - hinf) * dm_exp(-dt / htau);
     if (m_val < 0.0f) m_val = 0.0f;
