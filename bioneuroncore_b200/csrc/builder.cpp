@@ -383,6 +383,91 @@ void hostnet_from_aos(const BncBionData& aos, HostNet* hn) {
 
 namespace {
 
+// Lays a network of trees out for k_diffusion_tree: every component acyclic, of at most
+// 2,048 segments with at most kTreeMaxInc connections each, all intracellular.  Returns the
+// slots per tile (0: the tile kernels run it).
+struct TreeLayout {
+    std::vector<uint32_t> beg;
+    std::vector<uint16_t> par, grp;
+    std::vector<uint2> oth;
+    std::vector<float> area, dist;
+    uint32_t inc = 0;   // most connections of a segment
+};
+constexpr uint32_t kTreeMaxInc = 4;
+
+uint32_t tree_layout(const HostNet& hn, const std::vector<uint32_t>& conn_ok, const std::vector<uint32_t>& inv,
+                     const std::vector<uint32_t>& comp_beg, uint32_t n, TreeLayout* L) {
+    if (conn_ok.empty()) return 0;
+    uint32_t longest = 0;
+    std::vector<uint32_t> comp_at(n);   // first device segment of each segment's component
+    size_t nc = 0;
+    while (comp_beg[nc] < n) {
+        for (uint32_t i = comp_beg[nc]; i < comp_beg[nc + 1]; i++) comp_at[i] = comp_beg[nc];
+        longest = std::max(longest, comp_beg[nc + 1] - comp_beg[nc]);
+        nc++;
+    }
+    if (longest > 2048 || conn_ok.size() + nc != n) return 0;   // too large, or some component holds a cycle
+    // connections of each segment in connection order, a-role before b-role
+    std::vector<uint32_t> nb((size_t)n * kTreeMaxInc, UINT32_MAX), ne((size_t)n * kTreeMaxInc, UINT32_MAX);
+    std::vector<uint8_t> deg(n, 0);
+    for (uint32_t c : conn_ok) {
+        const auto& cn = hn.conn[c];
+        const uint32_t a = inv[cn.segment_a], b = inv[cn.segment_b];
+        if (a == b || !cn.is_intracellular || deg[a] == kTreeMaxInc || deg[b] == kTreeMaxInc) return 0;
+        nb[(size_t)a * kTreeMaxInc + deg[a]] = b; ne[(size_t)a * kTreeMaxInc + deg[a]++] = c;
+        nb[(size_t)b * kTreeMaxInc + deg[b]] = a; ne[(size_t)b * kTreeMaxInc + deg[b]++] = c;
+    }
+    for (uint32_t i = 0; i < n; i++) L->inc = std::max<uint32_t>(L->inc, deg[i]);
+    // tiles of whole components: the smallest capacity that holds the largest, from 512
+    const uint32_t cap = longest <= 512 ? 512 : longest <= 1024 ? 1024 : 2048;
+    L->beg.assign(1, 0);
+    for (size_t k = 0; k < nc; k++)
+        if (comp_beg[k + 1] - L->beg.back() > cap) L->beg.push_back(comp_beg[k]);
+    L->beg.push_back(n);
+    L->par.assign(n, 0xFFFF);
+    L->grp.assign(n, 0);
+    L->oth.assign(n, make_uint2(0xFFFFFFFFu, 0xFFFFFFFFu));
+    L->area.assign(n, 0.0f);
+    L->dist.assign(n, 1.0f);
+    std::vector<uint32_t> queue;
+    std::vector<uint8_t> seen(n, 0);
+    for (size_t t = 0; t + 1 < L->beg.size(); t++) {
+        const uint32_t s0 = L->beg[t], s1 = L->beg[t + 1];
+        uint32_t group = 0;
+        for (uint32_t i = s0; i < s1; i++) {
+            if (comp_at[i] == i && i != s0) group++;
+            L->grp[i] = (uint16_t)(group | (comp_at[i] == i ? 0x8000u : 0u));
+            uint32_t o[kTreeMaxInc];
+            for (uint32_t k = 0; k < kTreeMaxInc; k++) o[k] = k < deg[i] ? nb[(size_t)i * kTreeMaxInc + k] - s0 : 0xFFFFu;
+            L->oth[i] = make_uint2(o[0] | o[1] << 16, o[2] | o[3] << 16);
+            if (seen[i]) continue;
+            seen[i] = 1;   // the root of its component: parents breadth first from it
+            queue.assign(1, i);
+            for (size_t h = 0; h < queue.size(); h++) {
+                const uint32_t x = queue[h];
+                for (uint32_t k = 0; k < deg[x]; k++) {
+                    const uint32_t y = nb[(size_t)x * kTreeMaxInc + k];
+                    if (seen[y]) continue;
+                    seen[y] = 1;
+                    L->par[y] = (uint16_t)(x - s0);
+                    const auto& cn = hn.conn[ne[(size_t)x * kTreeMaxInc + k]];
+                    const SegLite &A = hn.seg[cn.segment_a], &B = hn.seg[cn.segment_b];
+                    const float r_min = A.radius < B.radius ? A.radius : B.radius;
+                    float area = 3.14159265f * r_min * r_min;
+                    if (area < 1e-6f) area = 1e-6f;
+                    float dist = (A.length + B.length) * 0.5f;
+                    if (dist < 0.1f) dist = 0.1f;
+                    L->area[y] = area;
+                    L->dist[y] = dist;
+                    queue.push_back(y);
+                }
+            }
+        }
+        if (group >= 2048) return 0;
+    }
+    return cap;
+}
+
 // Lays an unbranched network out for k_diffusion_path: every component a path of at most
 // 128 segments whose connections are all intracellular.  Returns the slots per lane, 0
 // when the network is not of that kind (the CTA-tile kernel runs it).
@@ -821,6 +906,12 @@ int build_network(const HostNet& hn, const Stimuli& stim, NetDev* dev, NetHost* 
     std::vector<float> pt_area, pt_dist;
     host->path_slots = opt.group_barriers ? path_layout(n, T, host->cluster, tile_seg_beg, tile_edge_beg, e_a, e_b, e_intra,
                                                         e_area, e_dist, &pt_seg, &pt_area, &pt_dist) : 0;
+    // ---- other networks of trees: the tiles of k_diffusion_tree (an explicit tile size or
+    // CTA barriers keep the tile kernels) ----
+    TreeLayout tree;
+    host->tree_slots = !host->path_slots && opt.group_barriers && opt.tile_segs == (uint32_t)kMaxTileSegs
+                           ? tree_layout(hn, conn_ok, host->inv, comp_members_off, n, &tree) : 0;
+    host->tree_inc = tree.inc;
     lap("edges");
     // incidence lists per device segment: the connections of its own tile that touch
     // it, in original connection order, a-role before b-role
@@ -1656,6 +1747,7 @@ int build_network(const HostNet& hn, const Stimuli& stim, NetDev* dev, NetHost* 
     int rc = BNC_OK;
     dev->n_seg = n; dev->n_tiles = T; dev->n_items = NI; dev->n_phases = n_phases;
     dev->n_syn = K; dev->n_rec = NR; dev->n_edges = E;
+    dev->n_tr = host->tree_slots ? (uint32_t)tree.beg.size() - 1u : 0u;
     dev->n_pt = host->path_slots ? (uint32_t)(pt_seg.size() / (32 * host->path_slots)) : 0u;
     uint32_t flags = 0;
     if (!conn_ok.empty()) flags |= NF_DIFFUSION;
@@ -1705,6 +1797,14 @@ int build_network(const HostNet& hn, const Stimuli& stim, NetDev* dev, NetHost* 
             dev->pt_seg = up(allocs, pt_seg, &rc);
             dev->pt_area = up(allocs, pt_area, &rc);
             dev->pt_dist = up(allocs, pt_dist, &rc);
+        }
+        if (host->tree_slots) {
+            dev->tr_beg = up(allocs, tree.beg, &rc);
+            dev->tr_par = up(allocs, tree.par, &rc);
+            dev->tr_oth = up(allocs, tree.oth, &rc);
+            dev->tr_area = up(allocs, tree.area, &rc);
+            dev->tr_dist = up(allocs, tree.dist, &rc);
+            dev->tr_grp = up(allocs, tree.grp, &rc);
         }
         dev->e_a = up(allocs, e_a, &rc);
         dev->e_b = up(allocs, e_b, &rc);

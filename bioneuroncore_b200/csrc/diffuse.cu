@@ -1053,6 +1053,7 @@ k_diffusion(NetDev d, float dt, unsigned long long tick, uint32_t S, uint32_t E)
 }
 
 #include "diffuse_path.cuh"
+#include "diffuse_tree.cuh"
 
 size_t diffusion_smem_bytes(uint32_t max_segs, uint32_t max_edges) {
     return diff_layout(max_segs, max_edges, nullptr, nullptr);
@@ -1074,6 +1075,10 @@ cudaError_t prepare_diffusion(const NetHost& host, cudaStream_t stream) {
         if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
         if (e != cudaSuccess) return e;
         g_ntd_ready[dev] = true;
+    }
+    if (host.tree_slots) {
+        e = host.tree_slots == 512 ? prepare_tree<512>() : (host.tree_slots == 1024 ? prepare_tree<1024>() : prepare_tree<2048>());
+        if (e != cudaSuccess) return e;
     }
     const size_t smem = diffusion_smem_bytes(host.max_tile_stride, host.max_tile_edges);
     if (smem > 48 * 1024) {
@@ -1125,6 +1130,7 @@ cudaError_t enqueue_diffusion(const NetDev& dev, const NetHost& host, float dt, 
         if (e != cudaSuccess) return e;
     }
     if (host.path_slots && dev.diff_mode == 0u) return launch_diffusion_path(dev, host.path_slots, dt, tick, stream);
+    if (host.tree_slots) return launch_diffusion_tree(dev, host.tree_slots, host.tree_inc, dt, tick, stream);
     const uint32_t S = host.max_tile_stride, E = host.max_tile_edges;
     const size_t smem = diffusion_smem_bytes(S, E);
     const uint32_t threads = std::max(host.diff_threads, diffusion_threads(host.max_tile_segs));

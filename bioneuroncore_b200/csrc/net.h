@@ -95,6 +95,18 @@ struct NetDev {
     float* pt_area;
     float* pt_dist;
     uint32_t n_pt;            // warps
+    // networks of trees (NetHost::tree_slots nonzero): tiles of k_diffusion_tree, whole
+    // components of consecutive segments, at most tree_slots each.  Per segment its parent
+    // (tile-local, 0xFFFF: none) with the contact area and length of that connection, the
+    // other ends of its connections in connection order (tile-local, 4 x 16 bits, 0xFFFF:
+    // none), and its convergence group as seg_grp has it
+    uint32_t* tr_beg;         // [n_tr + 1] (nullptr otherwise)
+    uint16_t* tr_par;
+    uint2* tr_oth;
+    float* tr_area;
+    float* tr_dist;
+    uint16_t* tr_grp;
+    uint32_t n_tr;            // tiles
     // edges (tile-grouped, tile-local endpoints)
     uint16_t* e_a;
     uint16_t* e_b;
@@ -301,6 +313,8 @@ struct NetHost {
     uint32_t max_tile_stride = 0;            // own + ghost segments of the largest tile
     uint32_t cluster = 1;                    // CTAs per diffusion cluster (2: tiles in pairs)
     uint32_t diff_threads = 32;              // threads per diffusion CTA
+    uint32_t tree_slots = 0;                 // slots per tile of k_diffusion_tree (0: not a network of trees)
+    uint32_t tree_inc = 0;                   // its segments' connections, at most
     uint32_t path_slots = 0;                 // slots per lane of k_diffusion_path (0: not an unbranched network)
     uint32_t diff_gm = 0;                    // diffusion barrier groups: 0 (CTA), 32 or 64 threads
     uint32_t group_tiles_32 = 0, group_tiles_64 = 0;   // tiles with warp / 64-thread barrier groups
