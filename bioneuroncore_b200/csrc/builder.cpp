@@ -429,43 +429,46 @@ uint32_t tree_layout(const HostNet& hn, const std::vector<uint32_t>& conn_ok, co
     L->oth.assign(n, make_uint2(0xFFFFFFFFu, 0xFFFFFFFFu));
     L->area.assign(n, 0.0f);
     L->dist.assign(n, 1.0f);
-    std::vector<uint32_t> queue;
     std::vector<uint8_t> seen(n, 0);
-    for (size_t t = 0; t + 1 < L->beg.size(); t++) {
-        const uint32_t s0 = L->beg[t], s1 = L->beg[t + 1];
-        uint32_t group = 0;
-        for (uint32_t i = s0; i < s1; i++) {
-            if (comp_at[i] == i && i != s0) group++;
-            L->grp[i] = (uint16_t)(group | (comp_at[i] == i ? 0x8000u : 0u));
-            uint32_t o[kTreeMaxInc];
-            for (uint32_t k = 0; k < kTreeMaxInc; k++) o[k] = k < deg[i] ? nb[(size_t)i * kTreeMaxInc + k] - s0 : 0xFFFFu;
-            L->oth[i] = make_uint2(o[0] | o[1] << 16, o[2] | o[3] << 16);
-            if (seen[i]) continue;
-            seen[i] = 1;   // the root of its component: parents breadth first from it
-            queue.assign(1, i);
-            for (size_t h = 0; h < queue.size(); h++) {
-                const uint32_t x = queue[h];
-                for (uint32_t k = 0; k < deg[x]; k++) {
-                    const uint32_t y = nb[(size_t)x * kTreeMaxInc + k];
-                    if (seen[y]) continue;
-                    seen[y] = 1;
-                    L->par[y] = (uint16_t)(x - s0);
-                    const auto& cn = hn.conn[ne[(size_t)x * kTreeMaxInc + k]];
-                    const SegLite &A = hn.seg[cn.segment_a], &B = hn.seg[cn.segment_b];
-                    const float r_min = A.radius < B.radius ? A.radius : B.radius;
-                    float area = 3.14159265f * r_min * r_min;
-                    if (area < 1e-6f) area = 1e-6f;
-                    float dist = (A.length + B.length) * 0.5f;
-                    if (dist < 0.1f) dist = 0.1f;
-                    L->area[y] = area;
-                    L->dist[y] = dist;
-                    queue.push_back(y);
+    std::atomic<bool> fits{true};
+    parallel_for(L->beg.size() - 1, [&](size_t t0, size_t t1) {
+        std::vector<uint32_t> queue;
+        for (size_t t = t0; t < t1; t++) {
+            const uint32_t s0 = L->beg[t], s1 = L->beg[t + 1];
+            uint32_t group = 0;
+            for (uint32_t i = s0; i < s1; i++) {
+                if (comp_at[i] == i && i != s0) group++;
+                L->grp[i] = (uint16_t)(group | (comp_at[i] == i ? 0x8000u : 0u));
+                uint32_t o[kTreeMaxInc];
+                for (uint32_t k = 0; k < kTreeMaxInc; k++) o[k] = k < deg[i] ? nb[(size_t)i * kTreeMaxInc + k] - s0 : 0xFFFFu;
+                L->oth[i] = make_uint2(o[0] | o[1] << 16, o[2] | o[3] << 16);
+                if (seen[i]) continue;
+                seen[i] = 1;   // the root of its component: parents breadth first from it
+                queue.assign(1, i);
+                for (size_t h = 0; h < queue.size(); h++) {
+                    const uint32_t x = queue[h];
+                    for (uint32_t k = 0; k < deg[x]; k++) {
+                        const uint32_t y = nb[(size_t)x * kTreeMaxInc + k];
+                        if (seen[y]) continue;
+                        seen[y] = 1;
+                        L->par[y] = (uint16_t)(x - s0);
+                        const auto& cn = hn.conn[ne[(size_t)x * kTreeMaxInc + k]];
+                        const SegLite &A = hn.seg[cn.segment_a], &B = hn.seg[cn.segment_b];
+                        const float r_min = A.radius < B.radius ? A.radius : B.radius;
+                        float area = 3.14159265f * r_min * r_min;
+                        if (area < 1e-6f) area = 1e-6f;
+                        float dist = (A.length + B.length) * 0.5f;
+                        if (dist < 0.1f) dist = 0.1f;
+                        L->area[y] = area;
+                        L->dist[y] = dist;
+                        queue.push_back(y);
+                    }
                 }
             }
+            if (group >= 2048) fits = false;
         }
-        if (group >= 2048) return 0;
-    }
-    return cap;
+    }, 16);
+    return fits ? cap : 0;
 }
 
 // Lays an unbranched network out for k_diffusion_path: every component a path of at most
@@ -947,7 +950,7 @@ int build_network(const HostNet& hn, const Stimuli& stim, NetDev* dev, NetHost* 
         std::vector<uint32_t> idx;
         for (uint32_t d = 0; d < n; d++) {
             uint32_t b = inc_off[d], e = inc_off[d + 1];
-            if (e - b < 2) continue;
+            if (e - b < 2 || std::is_sorted(key.begin() + b, key.begin() + e)) continue;   // tiles list them in order
             idx.resize(e - b);
             std::iota(idx.begin(), idx.end(), b);
             std::sort(idx.begin(), idx.end(), [&](uint32_t x, uint32_t y) { return key[x] < key[y]; });
