@@ -383,6 +383,39 @@ void hostnet_from_aos(const BncBionData& aos, HostNet* hn) {
 
 namespace {
 
+// The distinct lists of active types among the segments and each segment's list; false
+// when there are more than `most`.
+bool distinct_lists(uint32_t n, const std::vector<uint32_t>& off, const HostVec<uint8_t>& type, uint32_t most,
+                    HostVec<uint32_t>* list_of, std::vector<std::vector<uint8_t>>* lists) {
+    struct Part { size_t i0, i1; std::vector<uint32_t> global; };
+    std::vector<Part> parts;
+    std::mutex mu;
+    std::atomic<bool> few{true};
+    auto find = [](std::vector<std::vector<uint8_t>>& v, const uint8_t* b, const uint8_t* e) {
+        uint32_t x = 0;
+        while (x < v.size() && !(v[x].size() == (size_t)(e - b) && std::equal(b, e, v[x].begin()))) x++;
+        if (x == v.size()) v.emplace_back(b, e);
+        return x;
+    };
+    parallel_for(n, [&](size_t i0, size_t i1) {
+        std::vector<std::vector<uint8_t>> own;
+        for (size_t i = i0; i < i1 && few; i++) {
+            (*list_of)[i] = find(own, type.data() + off[i], type.data() + off[i + 1]);
+            if (own.size() > most) few = false;
+        }
+        if (!few) return;
+        std::lock_guard<std::mutex> lock(mu);
+        parts.push_back({i0, i1, {}});
+        for (const auto& l : own) parts.back().global.push_back(find(*lists, l.data(), l.data() + l.size()));
+    });
+    if (!few || lists->size() > most) return false;
+    parallel_for(parts.size(), [&](size_t p0, size_t p1) {
+        for (size_t p = p0; p < p1; p++)
+            for (size_t i = parts[p].i0; i < parts[p].i1; i++) (*list_of)[i] = parts[p].global[(*list_of)[i]];
+    }, 1);
+    return true;
+}
+
 // Lays a network of trees out for k_diffusion_tree: every component acyclic, of at most
 // 2,048 segments with at most kTreeMaxInc connections each, all intracellular.  Returns the
 // slots per tile (0: the tile kernels run it).
@@ -1006,8 +1039,24 @@ int build_network(const HostNet& hn, const Stimuli& stim, NetDev* dev, NetHost* 
         }
     });
     lap("active lists");
+    // ---- networks of few modifier lists: the whole list in one launch ----
+    // When segments share a few lists of active types (a cell type's soma, dendrites and
+    // axon), rows sorted by list keep all but the warps at a list's end on one model per
+    // item, however deep the group, so the phases of the whole list form one group.
+    const uint32_t chunk_segs = opt.chunk_segs ? std::min(opt.chunk_segs, n) : n;
+    HostVec<uint32_t> list_of(n);                     // list of each original segment
+    std::vector<std::vector<uint8_t>> lists;
+    bool by_list = opt.fuse_adaptive && opt.phase_cap == 0 && chunk_segs == n && max_active >= 2 && max_active <= kMaxFuse;
+    if (by_list) {
+        const uint32_t most = std::min(std::max(kMinWholeLists, n / kSegsPerWholeList), kMaxWholeLists);
+        by_list = distinct_lists(n, act_off, act_type, most, &list_of, &lists);
+        for (const auto& l : lists)
+            for (uint8_t t : l) by_list = by_list && !user_type[t];
+    }
     uint32_t n_phases = 0;
-    {
+    if (by_list) {
+        n_phases = max_active;
+    } else {
         std::vector<uint32_t> ptr(n, 0);
         uint64_t remaining = act_slot.size();
         std::vector<uint64_t> count(256);
@@ -1057,13 +1106,28 @@ int build_network(const HostNet& hn, const Stimuli& stim, NetDev* dev, NetHost* 
     struct ItemKey { uint16_t phase; uint8_t type; uint32_t dseg; uint32_t k; };
     // Items are bucketed by (chunk, phase): a chunk is a run of chunk_segs segments whose
     // step-1 records stay resident in L2 while all phases of the chunk run.
-    const uint32_t chunk_segs = opt.chunk_segs ? std::min(opt.chunk_segs, n) : n;
     const uint32_t n_chunks = (n + chunk_segs - 1) / chunk_segs;
     host->chunk_segs = chunk_segs;
     host->n_chunks = n_chunks;
     const size_t NB = (size_t)n_chunks * n_phases;
     std::vector<uint32_t> bucket_off(NB + 1, 0);
-    for (uint32_t d = 0; d < n; d++) {
+    std::vector<uint32_t> list_row;   // rows of each list: most items first, then by types
+    if (by_list) {
+        std::vector<uint32_t> count(lists.size(), 0), order(lists.size());
+        for (uint32_t i = 0; i < n; i++) count[list_of[i]]++;
+        std::iota(order.begin(), order.end(), 0u);
+        std::sort(order.begin(), order.end(), [&](uint32_t x, uint32_t y) {
+            return lists[x].size() != lists[y].size() ? lists[x].size() > lists[y].size() : lists[x] < lists[y];
+        });
+        list_row.resize(lists.size());
+        uint32_t row = 0;
+        for (uint32_t x : order) {
+            list_row[x] = row;
+            row += count[x];
+            for (size_t j = 0; j < lists[x].size(); j++) bucket_off[j + 1] += count[x];
+        }
+    }
+    for (uint32_t d = 0; d < n && !by_list; d++) {
         uint32_t i = host->perm[d];
         for (uint32_t k = act_off[i]; k < act_off[i + 1]; k++)
             bucket_off[(size_t)(d / chunk_segs) * n_phases + item_phase[k] + 1]++;
@@ -1076,13 +1140,23 @@ int build_network(const HostNet& hn, const Stimuli& stim, NetDev* dev, NetHost* 
     // once rows are sorted by their item count, and item (row r, phase p0 + j) sits at
     // bucket_off[p0 + j] + r.  Rows are sorted by (count descending, the types of their
     // items) so that warps run one sequence of models.
-    uint32_t fuse = std::min<uint32_t>(std::max<uint32_t>(opt.fuse_phases, 1u), kMaxFuse);
+    uint32_t fuse = std::min<uint32_t>(std::max<uint32_t>(by_list ? n_phases : opt.fuse_phases, 1u), kMaxFuse);
     if (n_chunks != 1 || n_phases < 2) fuse = 1;
-    for (uint32_t i = 0; i < n && fuse > 1; i++)
+    for (uint32_t i = 0; i < n && fuse > 1 && !by_list; i++)
         for (uint32_t k = act_off[i]; k < act_off[i + 1]; k++)
             if (item_phase[k] != k - act_off[i] || user_type[act_type[k]]) { fuse = 1; break; }
     HostVec<ItemKey> keys(act_slot.size());
-    if (fuse > 1) {
+    if (by_list) {
+        HostVec<uint32_t> row(n);
+        for (uint32_t d = 0; d < n; d++) row[d] = list_row[list_of[host->perm[d]]]++;
+        parallel_for(n, [&](size_t d0, size_t d1) {
+            for (uint32_t d = (uint32_t)d0; d < (uint32_t)d1; d++) {
+                const uint32_t k0 = act_off[host->perm[d]], k1 = act_off[host->perm[d] + 1];
+                for (uint32_t j = 0; j < k1 - k0; j++)
+                    keys[bucket_off[j] + row[d]] = {(uint16_t)j, act_type[k0 + j], d, k0 + j};
+            }
+        });
+    } else if (fuse > 1) {
         uint32_t rank[256];
         uint32_t R = 0;
         {
@@ -1195,6 +1269,7 @@ int build_network(const HostNet& hn, const Stimuli& stim, NetDev* dev, NetHost* 
         }
     }
     host->fuse = fuse;
+    host->first_gathers = by_list && bucket_off[1] == n;   // every segment has a row
     lap("item sort");
     const uint32_t NI = (uint32_t)keys.size();
     std::vector<uint32_t> phase_off(bucket_off.begin(), bucket_off.end());

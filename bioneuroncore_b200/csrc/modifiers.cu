@@ -11,9 +11,10 @@
 //                SMs at any moment -- run few channel models at a time, which keeps the
 //                many models' code within the instruction caches.  Each dispatch case
 //                loads and stores only the record fields its model uses.
-//  k_phase_group the same phases four to a launch by default (slot-order schedules):
-//                one thread per segment runs its items of those phases on the record
-//                held in registers, so the record crosses HBM once per group.
+//  k_phase_group the same phases four to a launch by default (slot-order schedules), or
+//                all of them where segments share few modifier lists: one thread per
+//                segment runs its items of those phases on the record held in registers,
+//                so the record crosses HBM once per group.
 //  k_diffusion   (diffuse.cu) stimuli, step 2.5 electrodiffusion, the presynaptic record.
 //  k_synapse     (synapse.cu) steps 3 and 4.
 #define BNC_MATH_OUTLINE 1   // 26 channel models in one kernel: keep exp/log out of line
@@ -241,7 +242,13 @@ struct PhaseGroup {
 // 1,007 before the models' divisions by a volume, a time constant or a GHK denominator
 // became corrected products (physics.cuh).  Items loaded one ahead cost more registers
 // than the waiting they saved (1,080 us).
-template <bool kX>
+// kFirst: the group builds the record itself instead of reading k_gather's.  Only where
+// the whole list is one group (NetHost::first_gathers): its rows follow the device order
+// inside each list, so the reads of the segments' arrays coalesce.  Step 1 of the small
+// set, with one launch per phase / one group behind k_gather / one group alone: 55.8 /
+// 29.1 / 20.8 us at 2,048 segments, 590 / 362 / 326 at 1.92M.  The large set's rows follow
+// their types instead: 816 us behind k_gather, 980 alone.  Narrower CTAs gave nothing.
+template <bool kX, bool kFirst>
 __global__ void __launch_bounds__(256, BNC_GROUP_MIN_CTAS)
 k_phase_group(NetDev d, float dt, PhaseGroup grp) {
     const uint32_t q = blockIdx.x * blockDim.x + threadIdx.x;
@@ -251,15 +258,29 @@ k_phase_group(NetDev d, float dt, PhaseGroup grp) {
     const uint32_t g = d.it_seg[grp.off[0] + q];
     SegRec* r = d.rec + g;
     DSeg s;
-    s.V = r->V;
+    double itot = 0.0;
+    if (kFirst) {
+        s.V = d.V[g];
 #pragma unroll
-    for (int k = 0; k < 7; k++) { s.in[k] = r->in[k]; s.out[k] = r->out[k]; }
-    s.atp = r->atp;
-    s.area = r->area;
-    s.vol = r->vol;
+        for (int k = 0; k < 7; k++) {
+            s.in[k] = d.ion_in[(size_t)k * N + g];
+            s.out[k] = d.ion_out[(size_t)k * N + g];
+        }
+        s.atp = d.atp[g];
+        s.area = d.area[g];
+        s.vol = d.vol[g];
+        d.c21_cur[g] = d.cav21_static[g];
+    } else {
+        s.V = r->V;
+#pragma unroll
+        for (int k = 0; k < 7; k++) { s.in[k] = r->in[k]; s.out[k] = r->out[k]; }
+        s.atp = r->atp;
+        s.area = r->area;
+        s.vol = r->vol;
+        itot = r->itot;
+    }
     dp_seg_derived(s);
     ghk_mono_fill(s.gc, s.V);
-    double itot = r->itot;
 #pragma unroll 1
     for (uint32_t j = 0; j < grp.n; j++) {
         if (q >= grp.off[j + 1] - grp.off[j]) break;
@@ -293,6 +314,10 @@ k_phase_group(NetDev d, float dt, PhaseGroup grp) {
     for (int k = 0; k < 7; k++) { r->in[k] = s.in[k]; r->out[k] = s.out[k]; }
     r->atp = s.atp;
     r->itot = itot;
+    if (kFirst) {
+        r->area = s.area;
+        r->vol = s.vol;
+    }
 }
 
 static bool g_tables_ready[64] = {false};   // per device: constant memory is per context
@@ -361,7 +386,7 @@ static cudaError_t enqueue_modifiers(const NetDev& dev, const NetHost& host, flo
     size_t u = 0;
     for (uint32_t c = 0; c < C; c++) {
         const uint32_t s0 = c * cs, s1 = std::min(dev.n_seg, s0 + cs);
-        k_gather<<<(s1 - s0 + 255) / 256, 256, 0, stream>>>(dev, s0, s1);
+        if (!host.first_gathers) k_gather<<<(s1 - s0 + 255) / 256, 256, 0, stream>>>(dev, s0, s1);
         if (host.fuse > 1) {   // one chunk, no registered device modifiers (the builder's rule)
             for (uint32_t p0 = 0; p0 < P; p0 += host.fuse) {
                 PhaseGroup grp;
@@ -370,13 +395,15 @@ static cudaError_t enqueue_modifiers(const NetDev& dev, const NetHost& host, flo
                 const uint32_t rows = grp.off[1] - grp.off[0];
                 if (rows == 0) continue;
                 const dim3 gs((rows + 255) / 256);
-                if (grp.n == 1) {
+                if (p0 == 0 && host.first_gathers) {
+                    if (dev.model_extras) k_phase_group<true, true><<<gs, 256, 0, stream>>>(dev, dt, grp);
+                    else k_phase_group<false, true><<<gs, 256, 0, stream>>>(dev, dt, grp);
+                } else if (grp.n == 1) {
                     if (dev.model_extras) k_phase<true><<<gs, 256, 0, stream>>>(dev, dt, grp.off[0], grp.off[1]);
                     else k_phase<false><<<gs, 256, 0, stream>>>(dev, dt, grp.off[0], grp.off[1]);
-                } else if (dev.model_extras) {
-                    k_phase_group<true><<<gs, 256, 0, stream>>>(dev, dt, grp);
                 } else {
-                    k_phase_group<false><<<gs, 256, 0, stream>>>(dev, dt, grp);
+                    if (dev.model_extras) k_phase_group<true, false><<<gs, 256, 0, stream>>>(dev, dt, grp);
+                    else k_phase_group<false, false><<<gs, 256, 0, stream>>>(dev, dt, grp);
                 }
             }
             continue;
@@ -401,7 +428,7 @@ uint32_t modifier_launches(const NetDev& dev, const NetHost& host) {
     const uint32_t P = dev.n_phases;
     const uint32_t C = host.n_chunks ? host.n_chunks : 1;
     if (host.phase_off.size() < (size_t)C * P + 1) return 0;
-    uint32_t n = C;   // k_gather
+    uint32_t n = host.first_gathers ? 0 : C;   // k_gather
     if (host.fuse > 1) {
         for (uint32_t p0 = 0; p0 < P; p0 += host.fuse) n += host.phase_off[p0 + 1] > host.phase_off[p0] ? 1u : 0u;
         return n;

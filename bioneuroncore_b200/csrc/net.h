@@ -269,8 +269,9 @@ struct BuildOptions {
     // 6.4M-segment large set, step 1 per tick: 1 phase 7.8 ms; at 3.2M segments
     // 1: 3.94, 2: 2.89, 3: 2.40, 4: 2.15, 6: 2.43, 9: 4.97, 17: 19.5 ms (deeper groups
     // diverge: rows sorted by their items' types share fewer types further down).
+    // Networks of few modifier lists ignore this depth (kSegsPerWholeList).
     uint32_t fuse_phases = 4;
-    // Lower fuse_phases while the rows sorted for its groups leave warps on more than
+    // Run whole lists in one launch where segments share few, and lower fuse_phases while the rows sorted for its groups leave warps on more than
     // kMaxWarpTypes distinct models per item on average (an explicit fuse_phases option
     // turns this off).
     bool fuse_adaptive = true;
@@ -288,6 +289,15 @@ constexpr double kMaxWarpTypes = 1.3;
 // Below this many segments a modifier launch is a few microseconds of work, its count
 // matters more than divergence, and the requested depth is kept.
 constexpr uint32_t kAdaptiveFuseMinSegs = 1u << 16;
+// A network whose segments share at most one list of active modifier types per
+// kSegsPerWholeList segments (or kMinWholeLists lists) runs the whole list in one launch:
+// at most one warp in four then spans two lists.  Small networks gain with any lists, as
+// launches outweigh divergence (2 to 16 segments of the large set, all lists distinct: 56
+// to 139 us against 180 to 242 with a launch per phase, 125 to 160 in groups of 4); at
+// 16,384 segments of all-distinct lists one group takes 215 us, groups of 4 take 161.
+constexpr uint32_t kSegsPerWholeList = 128;
+constexpr uint32_t kMinWholeLists = 16;
+constexpr uint32_t kMaxWholeLists = 256;
 
 // k_diffusion_path takes its low-latency form up to this many warps (4 per scheduler:
 // 1,800 warps 64.5 us against 72.8, 6,539 warps 172 against 169, 20,000 warps 544 against
@@ -321,6 +331,7 @@ struct NetHost {
     std::vector<uint32_t> phase_off;         // item range of each (chunk, phase) bucket (host copy)
     uint32_t chunk_segs = 0, n_chunks = 1;   // modifier-pass chunks of consecutive segments
     uint32_t fuse = 1;                       // modifier phases per launch (item order follows)
+    bool first_gathers = false;              // the first phase group reads the segments itself (no k_gather)
     double warp_models = 1.0;                // mean distinct models per warp and item of a group
     uint8_t item_dyn_rows = 0;               // state words (bits) any item updates: the rows exported
     struct UserRange { uint32_t bucket, type, begin, end; const void* kernel; };
