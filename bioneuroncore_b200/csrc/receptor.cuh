@@ -114,7 +114,7 @@ __device__ __forceinline__ double receptor_current(const RecKind& K, DMod& m, DS
 // chain, and its latency bounds the synapse step of any network that does not fill the
 // chip many times over.  With the reciprocals a receptor is about 16 dependent FP64
 // operations (9 cycles each) in place of three full divisions (112 cycles each) among 25,
-// and RecStep runs all four receptor kinds without divergence.
+// and receptor_step runs all four receptor kinds without divergence.
 struct RecSeg {
     double A1, D1, y1, e1, o0, o1, o3;   // monovalent: out Na and K times e1, out Cl
     double A2, D2, y2, o2;               // divalent: out Ca times e2
@@ -178,21 +178,33 @@ __device__ __forceinline__ float rec_relax(float x, float to, float dt, double t
 __device__ __forceinline__ float rec_clamp(float x) { return x < 1e-9f ? 1e-9f : x; }
 
 // receptor_current for a default-conductance receptor of a segment whose RecSeg is ok, the
-// same operations in the same order; every lane of the warp takes part (`on`: this lane
-// has a receptor), so that lanes with different kinds run one instruction stream.  r_inf:
-// nt / (nt + EC50), also the desensitisation gate's target (K_desens is 0 for all kinds).
-// w: the desensitisation gate, for NMDA the inactivation gate.  Returns whether it holds;
-// nothing is changed in a lane where it does not (a value out of the range in which the
-// corrected quotients are the IEEE ones, or not finite).
-__device__ __forceinline__ bool receptor_step(const RecSeg& f, const RecK& K, int kind, bool on, float den, float area,
-                                              float& r, float& w, float (&in)[7], float dt, float r_inf, float mod_scale,
-                                              double& I) {
-    const bool an = kind >= 2, nmda = kind == 1;
-    bool ok = f.ok;
+// same operations in the same order, in three stages of which only the second is part of
+// the segment's chain.  Every lane of the warp takes part, so that lanes with different
+// kinds run one instruction stream.
+//
+// The gates.  r_inf: nt / (nt + EC50), also the desensitisation gate's target (K_desens is
+// 0 for all kinds).  w: the desensitisation gate, relaxed; for NMDA the inactivation gate,
+// left to rec_tail.  Returns whether the corrected quotients are the IEEE ones here.
+__device__ __forceinline__ bool rec_gates(const RecK& K, int kind, float r, float& w, float dt, float r_inf, float& rn,
+                                          float& open) {
+    const bool nmda = kind == 1;
     const bool up = r_inf > r;
-    const float rn = rec_relax(r, r_inf, dt, up ? K.rise : K.decay, up ? K.y_rise : K.y_decay, ok);
-    float wn = rec_relax(w, r_inf, dt, K.des, K.y_des, ok);
-    const float open = nmda ? rn : rn * (1.0f - wn);
+    bool ok = !nmda | (fabsf(w) < 1e30f);
+    rn = rec_relax(r, r_inf, dt, up ? K.rise : K.decay, up ? K.y_rise : K.y_decay, ok);
+    const float wn = rec_relax(w, r_inf, dt, K.des, K.y_des, ok);
+    open = nmda ? rn : rn * (1.0f - wn);
+    w = nmda ? w : wn;
+    return ok;
+}
+// The currents: the sum of inward ones (It, without NMDA's block) and the segment's ions;
+// ca: the intracellular Ca2+ it leaves.  Returns `ok` as long as the fast form holds;
+// nothing is changed in a lane where it does not (a value out of the range in which the
+// corrected quotients are the IEEE ones, or not finite).  kInline: the Ca2+ current in line
+// with the others, which shortens the chain; else only where some lane has an NMDA receptor.
+template <bool kInline>
+__device__ __forceinline__ bool rec_flux(const RecSeg& f, const RecK& K, int kind, bool ok, float den, float area,
+                                         float open, float (&in)[7], float dt, float mod_scale, double& It, float& ca) {
+    const bool an = kind >= 2, nmda = kind == 1;
     const double N = (double)den * area;
     const double n0 = an ? f.o3 - (double)in[3] * f.e1 : (double)in[0] - f.o0;
     const double f0 = rec_div(f.A1 * n0, f.D1, f.y1);
@@ -202,31 +214,60 @@ __device__ __forceinline__ bool receptor_step(const RecSeg& f, const RecK& K, in
     const double q0 = rec_div(I0 * dt, f.cpm, f.yc);
     const float c0 = rec_clamp((float)((double)(an ? in[3] : in[0]) - (an ? -q0 : q0)));
     const float c1 = rec_clamp((float)((double)in[1] - rec_div(I1 * dt, f.cpm, f.yc)));
-    double It = an ? I0 : I0 + I1;
+    It = an ? I0 : I0 + I1;
+    float c2 = rec_clamp(in[2]);
+    const bool any = kInline || __any_sync(0xFFFFFFFFu, ok & nmda);
     ok &= rec_in_range(I0) & (an | rec_in_range(I1));
-    float c2 = in[2];
-    if (__any_sync(0xFFFFFFFFu, on & nmda)) {
+    if (any) {
         const double f2 = rec_div(f.A2 * ((double)in[2] - f.o2), f.D2, f.y2);
         const double I2 = K.P2 * f2 * N * open * mod_scale * A_TO_PA;
-        if (nmda) {
-            It += I2;
-            ok &= rec_in_range(I2) & (fabsf(w) < 1e30f);
-            c2 = rec_clamp((float)((double)in[2] - 0.5 * rec_div(I2 * dt, f.cpm, f.yc)));
-            // dp_nmda_cdi_coagonist
-            const double Ca_uM = (double)c2 * MM_TO_UM;
-            const double cdi_inf = 1.0 - 0.8f * Ca_uM / (Ca_uM + 1.0f);
-            const bool fast = cdi_inf < (double)w;
-            wn = (float)((double)w + rec_div((cdi_inf - (double)w) * dt, fast ? 500.0 : 9000.0, fast ? 1.0 / 500.0 : 1.0 / 9000.0));
-            wn = wn < 0.0f ? 0.0f : (wn > 1.0f ? 1.0f : wn);
-            It = It * f.mg * ((double)wn * (10.0f / (10.0f + 1.0f)));
-        }
+        const float n2 = rec_clamp((float)((double)in[2] - 0.5 * rec_div(I2 * dt, f.cpm, f.yc)));
+        c2 = nmda ? n2 : c2;
+        It = nmda ? It + I2 : It;
+        ok &= !nmda | (rec_in_range(I2) & (n2 < 1e30f));
     }
-    I = -It;
-    if (on && ok) {
+    ca = c2;
+    if (ok) {   // with the clamp of the ions the receptor leaves alone
+        in[0] = an ? rec_clamp(in[0]) : c0;
+        in[1] = an ? rec_clamp(in[1]) : c1;
+        in[2] = c2;
+        in[3] = an ? c0 : rec_clamp(in[3]);
+    }
+    return ok;
+}
+// a / b rounded to nearest for b in [1, 1e34] and a below it in magnitude: Newton's
+// iteration for y = 1 / b rounded to nearest, then Markstein's correction.  In line and
+// without the general division's branch, so that it overlaps the next receptor's chain.
+__device__ __forceinline__ double rec_quot(double a, double b) {
+    double y;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
+#pragma unroll
+    for (int k = 0; k < 2; k++) y = __fma_rn(__fma_rn(-b, y, 1.0), y, y);
+    return rec_div(a, b, y);
+}
+// NMDA's Mg2+ block and inactivation (dp_nmda_cdi_coagonist) of the current It.
+__device__ __forceinline__ void rec_tail(const RecSeg& f, float ca, float& w, float dt, double& It) {
+    const double Ca_uM = (double)ca * MM_TO_UM;
+    const double cdi_inf = 1.0 - rec_quot(0.8f * Ca_uM, Ca_uM + 1.0f);
+    const bool fast = cdi_inf < (double)w;
+    const float wn = (float)((double)w + rec_div((cdi_inf - (double)w) * dt, fast ? 500.0 : 9000.0, fast ? 1.0 / 500.0 : 1.0 / 9000.0));
+    w = wn < 0.0f ? 0.0f : (wn > 1.0f ? 1.0f : wn);
+    It = It * f.mg * ((double)w * (10.0f / (10.0f + 1.0f)));
+}
+// The three in turn, for a receptor at a time (`on`: this lane has one).
+__device__ __forceinline__ bool receptor_step(const RecSeg& f, const RecK& K, int kind, bool on, float den, float area,
+                                              float& r, float& w, float (&in)[7], float dt, float r_inf, float mod_scale,
+                                              double& I) {
+    float rn, wn = w, open, ca;
+    bool ok = rec_gates(K, kind, r, wn, dt, r_inf, rn, open);
+    ok = rec_flux<true>(f, K, kind, ok & f.ok & on, den, area, open, in, dt, mod_scale, I, ca);
+    if (__any_sync(0xFFFFFFFFu, ok & (kind == 1))) {
+        if (kind == 1) rec_tail(f, ca, wn, dt, I);
+    }
+    I = -I;
+    if (ok) {
         r = rn;
         w = wn;
-        if (an) in[3] = c0;
-        else { in[0] = c0; in[1] = c1; in[2] = c2; }
     }
     return ok;
 }

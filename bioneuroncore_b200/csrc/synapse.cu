@@ -277,14 +277,23 @@ __device__ __forceinline__ void syn_in_load(SynIn& x, const NetDev& d, uint32_t 
     }
 }
 
-// 64 threads a CTA spread the first warps, which hold the longest chains, over the SMs;
-// 128 registers hold the pipeline (1.28M segments, steps 3 and 4: 445 us at 8 CTAs per
-// SM, 493 at 6, 518 at 10; 55k segments: 156, 142, 209; 756 and 545 before the chain was
-// shortened and its loads moved a step ahead).
+// 64 threads a CTA spread the first warps, which hold the longest chains, over the SMs.
+// Before the chain was shortened and its loads moved a step ahead, steps 3 and 4 took 756 us
+// at 1.28M segments and 545 at 55k.
 constexpr unsigned kSynThreads = 64;
+// Up to this many segments k_synapse takes the form for short chains of few warps (kFew),
+// from there on the one for many warps.  Steps 3 and 4 of the large set in the two forms:
+// 128k segments 116 us against 139, 256k 138 / 162, 384k 150 / 177, 512k 193 / 182,
+// 1.28M 468 / 448; the small set: 256k 34 / 36, 640k 58 / 53.
+constexpr uint32_t kSynFewSegs = 400000;
 
-template <bool kX>
-__global__ void __launch_bounds__(kSynThreads, 8)
+// kFew: 6 CTAs per SM with as many registers as the receptor loop wants, the Ca2+ current in
+// line with the others, and NMDA's tail one receptor late, beside the next one's currents.
+// A warp alone on its scheduler then takes about 390 instructions a receptor at 4.4 cycles
+// each; the 25,600 synapses of 256 64-segment neurons take 100 us instead of 118.  Not
+// kFew: 8 CTAs of 128 registers, and NMDA's parts only where a lane has such a receptor.
+template <bool kX, bool kFew>
+__global__ void __launch_bounds__(kSynThreads, kFew ? 6 : 8)
 k_synapse(NetDev d, float dt, unsigned long long tick, int first_tick) {
     __shared__ RecK rec_k[4];
     if (threadIdx.x < 4) rec_k_fill(rec_k[threadIdx.x], gRec[threadIdx.x]);
@@ -386,7 +395,17 @@ k_synapse(NetDev d, float dt, unsigned long long tick, int first_tick) {
         }
         // receptors (simulation_host.cpp:490-500), j-th receptors of the slice side by side
         float I_syn = 0.0f;
-        double I_rec = 0.0;
+        struct { double It; float ca, w; uint32_t r; bool on, nmda; } prev = {0.0, 0.0f, 0.0f, 0, false, false};
+        auto tail = [&]() {
+            double I = prev.It;
+            if (kFew || __any_sync(0xFFFFFFFFu, prev.nmda)) {
+                float w = prev.w;
+                rec_tail(rs, prev.ca, w, dt, I);
+                if (prev.nmda) d.rc_st[(size_t)2 * NR + prev.r] = w;
+                I = prev.nmda ? I : prev.It;
+            }
+            if (prev.on) I_syn = (float)(I_syn - I);
+        };
         const float ri_ampa = nt_glu / (nt_glu + 0.5f), ri_nmda = nt_glu / (nt_glu + 1.0f),
                     ri_gabaa = nt_gaba / (nt_gaba + 1.0f), ri_gly = nt_gly / (nt_gly + 0.5f);   // EC50 of each kind
         const uint32_t maxr = __reduce_max_sync(0xFFFFFFFFu, n_rc);
@@ -404,18 +423,25 @@ k_synapse(NetDev d, float dt, unsigned long long tick, int first_tick) {
             const bool on = n_rc > j;
             const int kind = receptor_kind(cur.type);
             const float parea = (post_area > 0.0f) ? post_area : s.area;
-            float r0 = cur.s0, w0 = kind == 1 ? cur.s2 : cur.s1;   // the state words the kind updates
-            const bool held = receptor_step(rs, rec_k[kind], kind, on && cur.av == 0, cur.den, parea, r0, w0, s.in, dt,
-                                            kind == 0 ? ri_ampa : kind == 1 ? ri_nmda : kind == 2 ? ri_gabaa : ri_gly,
-                                            scale, I_rec);
+            float rn, wn = kind == 1 ? cur.s2 : cur.s1, open;   // the state words the kind updates
+            const bool g = rec_gates(rec_k[kind], kind, cur.s0, wn, dt,
+                                     kind == 0 ? ri_ampa : kind == 1 ? ri_nmda : kind == 2 ? ri_gabaa : ri_gly, rn, open);
+            // the receptor before leaves the segment's chain here: its tail runs beside this one's currents
+            if (kFew) tail();
+            double It;
+            float ca;
+            const bool held = rec_flux<kFew>(rs, rec_k[kind], kind, g & rs.ok & on & (cur.av == 0), cur.den, parea, open, s.in,
+                                       dt, scale, It, ca);
+            prev.on = on;
+            prev.nmda = held & (kind == 1);
+            prev.It = It;
+            prev.ca = ca;
+            prev.w = wn;
+            prev.r = r;
             if (on) {
-                if (held && cur.av == 0) {
-                    if (!touched) {   // dp_clamp_ions of the ions the receptor left alone
-#pragma unroll
-                        for (int q = 0; q < 7; q++) s.in[q] = rec_clamp(s.in[q]);
-                    }
-                    d.rc_st[r] = r0;
-                    d.rc_st[(size_t)(kind == 1 ? 2 : 1) * NR + r] = w0;
+                if (held) {
+                    d.rc_st[r] = rn;
+                    if (kind != 1) d.rc_st[NR + r] = wn;
                 } else {
                     RecSlow x;
                     x.s = s;
@@ -429,15 +455,16 @@ k_synapse(NetDev d, float dt, unsigned long long tick, int first_tick) {
                     receptor_slow(&x, kind, dt, kind <= 1 ? nt_glu : (kind == 2 ? nt_gaba : nt_gly), scale);
 #pragma unroll
                     for (int q = 0; q < 7; q++) s.in[q] = x.s.in[q];
-                    I_rec = x.I;
+                    prev.It = -x.I;
                     d.rc_st[r] = x.m.st[0];
                     d.rc_st[(size_t)NR + r] = x.m.st[1];
                     d.rc_st[(size_t)2 * NR + r] = x.m.st[2];
                 }
-                I_syn = (float)(I_syn + I_rec);
-                touched = true;
             }
+            if (!kFew) tail();
         }
+        if (kFew) tail();
+        touched |= n_rc > 0;
         if (maxr == 0) {   // no receptor in this slice: the next one's first is still to load
             has = __ballot_sync(0xFFFFFFFFu, syn.n_rc > 0);
             if (syn.n_rc > 0) rec_in_load(rec, d, rbase + __popc(has & lt_mask));
@@ -567,9 +594,9 @@ k_synapse(NetDev d, float dt, unsigned long long tick, int first_tick) {
         if (V > 150.0f) V = 150.0f;
     }
     d.V[i] = V;
-    if (touched) {
+    if (touched) {   // the receptors' dp_clamp_ions
 #pragma unroll
-        for (int q = 0; q < 7; q++) d.ion_in[(size_t)q * N + i] = s.in[q];
+        for (int q = 0; q < 7; q++) d.ion_in[(size_t)q * N + i] = rec_clamp(s.in[q]);
     }
     if (syn_on) {
         const uint32_t mask = first_tick ? 0x7FFFu : d.nt_used_mask;
@@ -626,10 +653,15 @@ uint32_t synapse_launches(const NetDev& dev) {
 cudaError_t launch_synapse(const NetDev& dev, float dt, unsigned long long tick, int first_tick,
                            cudaStream_t stream) {
     const bool extras = dev.syn_extras != 0;
-    if (extras) k_synapse<true><<<(dev.n_seg + kSynThreads - 1) / kSynThreads, kSynThreads, 0, stream>>>(dev, dt, tick, first_tick);
-    else {
+    const bool few = dev.n_seg <= kSynFewSegs;
+    const unsigned grid = (dev.n_seg + kSynThreads - 1) / kSynThreads;
+    if (extras) {
+        if (few) k_synapse<true, true><<<grid, kSynThreads, 0, stream>>>(dev, dt, tick, first_tick);
+        else k_synapse<true, false><<<grid, kSynThreads, 0, stream>>>(dev, dt, tick, first_tick);
+    } else {
         if (dev.n_syn) k_release<<<(dev.n_syn + 255) / 256, 256, 0, stream>>>(dev, dt, tick);
-        k_synapse<false><<<(dev.n_seg + kSynThreads - 1) / kSynThreads, kSynThreads, 0, stream>>>(dev, dt, tick, first_tick);
+        if (few) k_synapse<false, true><<<grid, kSynThreads, 0, stream>>>(dev, dt, tick, first_tick);
+        else k_synapse<false, false><<<grid, kSynThreads, 0, stream>>>(dev, dt, tick, first_tick);
     }
     if (dev.gl_cap) k_glia<<<(dev.n_glia + 127) / 128, 128, 0, stream>>>(dev);
     if (dev.sy_gj) k_gj_commit<<<(dev.n_gj + 255) / 256 < 1184 ? (dev.n_gj + 255) / 256 : 1184, 256, 0, stream>>>(dev);
