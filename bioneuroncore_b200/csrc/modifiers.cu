@@ -247,7 +247,11 @@ struct PhaseGroup {
 // inside each list, so the reads of the segments' arrays coalesce.  Step 1 of the small
 // set, with one launch per phase / one group behind k_gather / one group alone: 55.8 /
 // 29.1 / 20.8 us at 2,048 segments, 590 / 362 / 326 at 1.92M.  The large set's rows follow
-// their types instead: 816 us behind k_gather, 980 alone.  Narrower CTAs gave nothing.
+// their types instead: 816 us behind k_gather, 980 alone.
+// CTAs of 128 threads: a group's last rows, the shortest and slowest to come, leave less of
+// an SM idle.  Ticks with 256 / 128 / 64 threads: large set 285 / 279 / 281 us at 16,384
+// segments, 356 / 347 / 347 at 55,537, 1,710 / 1,699 / 1,701 at 1.28M; small set 109 / 107 /
+// 105 at 115,200, but 1,116 / 1,124 / 1,127 at 1.92M, where 256 stay beyond one wave.
 template <bool kX, bool kFirst>
 __global__ void __launch_bounds__(256, BNC_GROUP_MIN_CTAS)
 k_phase_group(NetDev d, float dt, PhaseGroup grp) {
@@ -394,16 +398,17 @@ static cudaError_t enqueue_modifiers(const NetDev& dev, const NetHost& host, flo
                 for (uint32_t j = 0; j <= kMaxFuse; j++) grp.off[j] = host.phase_off[std::min(p0 + j, p0 + grp.n)];
                 const uint32_t rows = grp.off[1] - grp.off[0];
                 if (rows == 0) continue;
-                const dim3 gs((rows + 255) / 256);
+                const uint32_t T = rows > 4u * 256u * 148u && p0 == 0 && host.first_gathers ? 256 : 128;
+                const dim3 gs((rows + T - 1) / T);
                 if (p0 == 0 && host.first_gathers) {
-                    if (dev.model_extras) k_phase_group<true, true><<<gs, 256, 0, stream>>>(dev, dt, grp);
-                    else k_phase_group<false, true><<<gs, 256, 0, stream>>>(dev, dt, grp);
+                    if (dev.model_extras) k_phase_group<true, true><<<gs, T, 0, stream>>>(dev, dt, grp);
+                    else k_phase_group<false, true><<<gs, T, 0, stream>>>(dev, dt, grp);
                 } else if (grp.n == 1) {
-                    if (dev.model_extras) k_phase<true><<<gs, 256, 0, stream>>>(dev, dt, grp.off[0], grp.off[1]);
-                    else k_phase<false><<<gs, 256, 0, stream>>>(dev, dt, grp.off[0], grp.off[1]);
+                    if (dev.model_extras) k_phase<true><<<gs, T, 0, stream>>>(dev, dt, grp.off[0], grp.off[1]);
+                    else k_phase<false><<<gs, T, 0, stream>>>(dev, dt, grp.off[0], grp.off[1]);
                 } else {
-                    if (dev.model_extras) k_phase_group<true, false><<<gs, 256, 0, stream>>>(dev, dt, grp);
-                    else k_phase_group<false, false><<<gs, 256, 0, stream>>>(dev, dt, grp);
+                    if (dev.model_extras) k_phase_group<true, false><<<gs, T, 0, stream>>>(dev, dt, grp);
+                    else k_phase_group<false, false><<<gs, T, 0, stream>>>(dev, dt, grp);
                 }
             }
             continue;
