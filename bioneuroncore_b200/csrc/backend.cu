@@ -53,8 +53,10 @@ struct Backend {
         uint8_t* md_slot;     // release modulator -> autoreceptor slot
         uint32_t* gj_syn;     // gap junction -> record
     } xm{};
-    // Field reads: original -> device segment, and one field in original order (owned by
-    // allocs, made at the first read that needs them)
+    // Field reads: original -> device segment (null: the same order), and one field in
+    // original order (owned by allocs, made at load: a cudaMalloc in front of the first read
+    // of a loaded network took up to 23 ms; rd_mu: reads of several host threads)
+    std::mutex rd_mu;
     uint32_t* rd_inv = nullptr;
     float* rd_buf = nullptr;
     uint32_t tick_stride = 1;   // the tick counter's step per tick (2: the reference's batch mode)
@@ -651,6 +653,23 @@ static void apply_protein_mapping(BncBionData& d) {
     }
 }
 
+// What field reads need of a network just built; without memory for it they go through the
+// host (read_in_order).
+static void prepare_reads(Backend* b) {
+    const size_t bytes = (size_t)b->dev.n_seg * sizeof(uint32_t);
+    uint32_t* inv = nullptr;
+    if (!b->host.perm_identity) {
+        inv = static_cast<uint32_t*>(b->allocs.alloc(bytes));
+        if (!inv || cudaMemcpy(inv, b->host.inv.data(), bytes, cudaMemcpyHostToDevice) != cudaSuccess) {
+            cudaGetLastError();
+            return;
+        }
+    }
+    b->rd_buf = static_cast<float*>(b->allocs.alloc(bytes));
+    if (b->rd_buf) b->rd_inv = inv;
+    else cudaGetLastError();
+}
+
 static int load_common(Backend* b, BncBionData& aos, bool keep_aos) {
     cudaSetDevice(b->device);
     apply_protein_mapping(aos);
@@ -658,6 +677,7 @@ static int load_common(Backend* b, BncBionData& aos, bool keep_aos) {
     hostnet_from_aos(aos, &hn);
     int rc = build_network(hn, b->stim, &b->dev, &b->host, &b->allocs);
     if (rc != BNC_OK) { b->reset_network(); return rc; }
+    prepare_reads(b);
     if (keep_aos) { b->aos = aos; b->owns_aos = true; }
     b->loaded = true;
     if (keep_aos) return make_records_managed(b);
@@ -1125,6 +1145,7 @@ int bnc_load_generated_opts(void* sim, const BncNetgenParams* p, const BncBuildO
     cudaSetDevice(b->device);
     rc = build_network(hn, b->stim, &b->dev, &b->host, &b->allocs, to_options(o));
     if (rc != BNC_OK) { b->reset_network(); return rc; }
+    prepare_reads(b);
     b->loaded = true;
     return BNC_OK;
 }
@@ -1178,6 +1199,7 @@ static int load_members(Backend* b, const BncNetgenParams* members, uint32_t n_m
     cudaSetDevice(b->device);
     rc = build_network(hn, b->stim, &b->dev, &b->host, &b->allocs, opt);
     if (rc != BNC_OK) { b->reset_network(); return rc; }
+    prepare_reads(b);
     b->members = std::move(mem);
     b->loaded = true;
     return BNC_OK;
@@ -1284,6 +1306,7 @@ int bnc_load_ensemble_aos(void* sim, const BncBionData* members, const BncCurren
     cudaSetDevice(b->device);
     int rc = build_network(hn, b->stim, &b->dev, &b->host, &b->allocs);
     if (rc != BNC_OK) { b->reset_network(); return rc; }
+    prepare_reads(b);
     b->members = std::move(mem);
     b->loaded = true;
     return BNC_OK;
@@ -1487,16 +1510,9 @@ static int read_in_order(Backend* b, const float* src, const uint32_t* counts, f
     const uint32_t N = b->dev.n_seg;
     const size_t bytes = (size_t)N * sizeof(float);
     const bool identity = b->host.perm_identity;
+    std::unique_lock<std::mutex> lock(b->rd_mu, std::defer_lock);
     if (!identity || counts) {
-        if (!b->rd_buf) b->rd_buf = static_cast<float*>(b->allocs.alloc(bytes));
-        if (!identity && !b->rd_inv) {
-            b->rd_inv = static_cast<uint32_t*>(b->allocs.alloc((size_t)N * sizeof(uint32_t)));
-            if (b->rd_inv && cudaMemcpyAsync(b->rd_inv, b->host.inv.data(), (size_t)N * sizeof(uint32_t),
-                                             cudaMemcpyHostToDevice, b->stream) != cudaSuccess)
-                return cuda_fail(cudaGetLastError(), "read");
-        }
-        if (!b->rd_buf || (!identity && !b->rd_inv)) {   // no device memory left: in order on the host
-            cudaGetLastError();
+        if (!b->rd_buf) {   // the load left no device memory for it: in order on the host
             std::vector<uint32_t> v(N);
             int rc = sync_stream(b);
             if (rc != BNC_OK) return rc;
@@ -1511,7 +1527,8 @@ static int read_in_order(Backend* b, const float* src, const uint32_t* counts, f
             }
             return BNC_OK;
         }
-        k_read_field<<<(N + 255) / 256, 256, 0, b->stream>>>(src, counts, identity ? nullptr : b->rd_inv, b->rd_buf, N);
+        lock.lock();   // held until the copy out of rd_buf is done
+        k_read_field<<<(N + 255) / 256, 256, 0, b->stream>>>(src, counts, b->rd_inv, b->rd_buf, N);
         src = b->rd_buf;
     }
     const cudaError_t e = cudaMemcpyAsync(out, src, bytes, cudaMemcpyDeviceToHost, b->stream);

@@ -3,6 +3,8 @@ capacities and their edges, three and four connections per segment, connection l
 any order and direction, values out of the corrected quotients' range, the
 residual-controlled solves with the ion ledger, and trees that an explicit tile size keeps
 on the tile kernels.  All tests are marked gpu."""
+from concurrent.futures import ThreadPoolExecutor
+
 import numpy as np
 import pytest
 
@@ -97,3 +99,16 @@ def test_values_out_of_range():
 def test_explicit_tiles_keep_the_tile_kernels(depth, tile):
     _check(NetgenParams(family=NET_TREES, n_neurons=3, tree_depth=depth, seed=4, flags=NETGEN_PERTURB_IONS),
            options=BuildOptions(tile_segs=tile), steps=(1, 4))
+
+
+def test_field_reads_from_several_threads():
+    """reads of one handle on several host threads at once return what single reads return
+    (a field out of order passes through one device buffer of the handle)"""
+    gpu = Backend()
+    gpu.load_generated(NetgenParams(family=NET_TREES, n_neurons=24, tree_depth=9, seed=5, flags=NETGEN_PERTURB_IONS))
+    gpu.run_ticks(2, DT)
+    want = {f: np.asarray(gpu.segment_field(*f)).copy() for f in FIELDS}
+    with ThreadPoolExecutor(8) as pool:
+        got = list(pool.map(lambda f: (f, np.asarray(gpu.segment_field(*f))), FIELDS * 12))
+    for f, x in got:
+        assert np.array_equal(x.view(np.uint32), want[f].view(np.uint32)), "%s[%d]" % f
