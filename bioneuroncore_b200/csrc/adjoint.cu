@@ -32,7 +32,7 @@
 //
 // What bounds it: instruction issue behind latency (forward 43% of issue slots at 14 warps
 // per SM, backward 30% at 8, its 230 registers the limit).  64 neurons x 64 segments, 16
-// sets, 160 ticks: forward 42.2 -> 11.0 ms, backward 139.7 -> 67.0, by what the plain tick
+// sets, 160 ticks: forward 42.2 -> 11.0 ms, backward 139.7 -> 63.2, by what the plain tick
 // does too (one Bernoulli pair per valence, corrected quotients, a phi_e solve left at its
 // fixed point), the channel models in line, their items and each synapse's place in the
 // release log in shared memory, two-entry sweeps, and twice the forward CTAs per SM.
@@ -1349,9 +1349,11 @@ __device__ void tick_rev(const AdjDev& d, const Ctx& c, const Lay& L, const Scr&
         const float lIt = L.lI[tid];
         const uint32_t ni = c.nit;
         float lV = lam[tid];
+        const float cpv = (float)(adj::kF * c.vol / 1000.0);
         float nx[5];   // an item's recorded inputs, loaded one item ahead
 #pragma unroll
         for (int k = 0; k < 5; k++) nx[k] = ni ? sc.pre[((ni - 1) * 5 + k) * Sm + tid] : 0.0f;
+#pragma unroll 1
         for (int j = (int)ni - 1; j >= 0; j--) {
             constexpr uint32_t IS = ItemStride<kFull>::v;
             const uint32_t itw = L.itw[j * Sm + tid];
@@ -1384,15 +1386,14 @@ __device__ void tick_rev(const AdjDev& d, const Ctx& c, const Lay& L, const Scr&
                                  lam[(8 + ion) * Sm + tid],
                                  lIt};
             float lx[6];
-            if (type == 123) adj::vjp_kvdr_f(lo, lx, pV, pG0, pCi, pCo, den, c.area, c.vol, dt, pst);
-            else if (type == 107) adj::vjp_k2p_f(lo, lx, pV, pCi, pCo, den, c.area, c.vol, dt, pst);
-            else if (kFull && type == 1) {   // out of line, through arrays of its own (lo / lx stay in registers)
+            if (kFull && type == 1) {   // out of line, through arrays of its own (lo / lx stay in registers)
                 float lo1[6], lx1[6];
                 for (int k = 0; k < 6; k++) lo1[k] = lo[k];
                 adj::vjp_cav13(lo1, lx1, pV, pG0, pG1, pCi, pCo, den, c.area, c.vol, dt, pst);
                 for (int k = 0; k < 6; k++) lx[k] = lx1[k];
             }
-            else adj::vjp_nav_f(lo, lx, pV, pG0, pG1, pCi, pCo, den, c.area, c.vol, dt, type == 142 ? 1 : 0, pst[5]);
+            else adj::vjp_item_f(type, lo, lx, pV, pG0, pG1, pCi, pCo, den, c.area, cpv, dt,
+                                 (itw >> 16) ? nullptr : pst);
             lV = lx[0];
             if (ng > 0) lam[(15 + go) * Sm + tid] = lx[1];
             if (ng > 1) lam[(16 + go) * Sm + tid] = lx[2];

@@ -637,61 +637,67 @@ __device__ __noinline__ void vjp_pump(float* lp, float V, float Na, float Ko, fl
     lp[5] = la1 + lx[3];
 }
 
-__device__ __forceinline__ void vjp_nav_f(const float* lo, float* lx, float V0, float m0, float h0, float cin, float cout,
-                                          float den, float area, double vol, float dt, int is12, float ttx) {
-    const bool mV = V0 >= -200.0f && V0 <= 200.0f;
-    const float V = mV ? V0 : (V0 < -200.0f ? -200.0f : 200.0f);
+// vtrap_f out of line, for callers that evaluate several: (value, derivative)
+__device__ __noinline__ float2 vtrap_call(float x, float y) {
+    float2 r;
+    vtrap_f(x, y, &r.x, &r.y);
+    return r;
+}
+
+// A channel's gates as its vector-Jacobian product needs them: the open probability and its
+// partials by the (clamped) gates, the gates' partials by V and by themselves, and the
+// permeability times the area.
+struct GateF {
+    float V, open, Kc;
+    float do0, do1, d0V, d1V, d00, d11;
+};
+__device__ __forceinline__ GateF nav_gates_f(float V0, float m0, float h0, float area, float dt, int is12, float ttx) {
+    GateF g;
+    const float V = V0 >= -200.0f && V0 <= 200.0f ? V0 : (V0 < -200.0f ? -200.0f : 200.0f);
+    g.V = V;
     const float cam = is12 ? 23.0f : 43.0f, cah = is12 ? 41.5f : 50.0f, cbh = is12 ? 66.5f : 75.0f,
                 chh = is12 ? 63.5f : 72.0f;
-    float am, dam, bm, dbm, ah, dah, bh, dbh;
-    vtrap_f(V + cam, 6.0f, &am, &dam); am *= 0.182f; dam *= 0.182f;
-    vtrap_f(-(V + cam), 6.0f, &bm, &dbm); bm *= 0.124f; dbm *= -0.124f;
-    vtrap_f(V + cah, 5.0f, &ah, &dah); ah *= 0.024f; dah *= 0.024f;
-    vtrap_f(-(V + cbh), 5.0f, &bh, &dbh); bh *= 0.0091f; dbh *= -0.0091f;
+    const float2 ta = vtrap_call(V + cam, 6.0f), tb = vtrap_call(-(V + cam), 6.0f);
+    const float2 tc = vtrap_call(V + cah, 5.0f), td = vtrap_call(-(V + cbh), 5.0f);
+    const float am = ta.x * 0.182f, dam = ta.y * 0.182f, bm = tb.x * 0.124f, dbm = tb.y * -0.124f;
+    const float ah = tc.x * 0.024f, dah = tc.y * 0.024f, bh = td.x * 0.0091f, dbh = td.y * -0.0091f;
     const float sm = am + bm, sh = ah + bh;
     const float minf = am / sm, dminf = (dam * bm - am * dbm) / (sm * sm);
-    const float mtau = 1.0f / sm, dmtau = -(dam + dbm) / (sm * sm);
     float hinf, dhinf;
     logistic_f((V + chh) / 6.2f, &hinf, &dhinf);
     dhinf /= 6.2f;
-    const float htau = 1.0f / sh, dhtau = -(dah + dbh) / (sh * sh);
-    const float Em = expf(-dt / mtau), dEm = Em * dt / (mtau * mtau) * dmtau;
-    const float Eh = expf(-dt / htau), dEh = Eh * dt / (htau * htau) * dhtau;
-    const float mu_ = minf + (m0 - minf) * Em, hu_ = hinf + (h0 - hinf) * Eh;
-    const bool mm = mu_ >= 0.0f && mu_ <= 1.0f, mh = hu_ >= 0.0f && hu_ <= 1.0f;
-    const float mv = mm ? mu_ : (mu_ < 0.0f ? 0.0f : 1.0f), hv = mh ? hu_ : (hu_ < 0.0f ? 0.0f : 1.0f);
-    const float dm_dV = mm ? dminf * (1.0f - Em) + (m0 - minf) * dEm : 0.0f;
-    const float dh_dV = mh ? dhinf * (1.0f - Eh) + (h0 - hinf) * dEh : 0.0f;
-    const float dm_dm = mm ? Em : 0.0f, dh_dh = mh ? Eh : 0.0f;
+    // the gates x -> inf + (x - inf) e^(-dt / tau), tau = 1 / sum
+    float u[2], dV[2], e[2];
+#pragma unroll 1
+    for (int k = 0; k < 2; k++) {
+        const float sum = k ? sh : sm, inf = k ? hinf : minf, dinf = k ? dhinf : dminf, x0 = k ? h0 : m0;
+        const float tau = 1.0f / sum, dtau = -(k ? dah + dbh : dam + dbm) / (sum * sum);
+        const float E = expf(-dt / tau), dE = E * dt / (tau * tau) * dtau;
+        const float w = inf + (x0 - inf) * E;
+        const bool in = w >= 0.0f && w <= 1.0f;
+        const float uv = in ? w : (w < 0.0f ? 0.0f : 1.0f), dVv = in ? dinf * (1.0f - E) + (x0 - inf) * dE : 0.0f,
+                    ev = in ? E : 0.0f;
+        if (k) { u[1] = uv; dV[1] = dVv; e[1] = ev; }
+        else { u[0] = uv; dV[0] = dVv; e[0] = ev; }
+    }
+    g.d0V = dV[0]; g.d1V = dV[1]; g.d00 = e[0]; g.d11 = e[1];
+    const float mv = u[0], hv = u[1];
     const float cdiv = 1.0f + (ttx > 0.0f ? ttx : 0.0f) / (is12 ? 10.0f : 5.0f);
-    const float open = mv * mv * mv * hv / cdiv;
-    const float do_dm = 3.0f * mv * mv * hv / cdiv, do_dh = mv * mv * mv / cdiv;
-    const float gamma = is12 ? 20.8f : 20.7f;
-    const float Kc = (float)((double)gamma * 1e-12 * (kR * kT) / (kF * kF * (double)55.964f) * 1e12) * area;
-    const GhkF G = ghk_mono_f(V, cin, cout);
-    const float I = Kc * G.F * den * open;
-    const float cpv = (float)(kF * vol / 1000.0);
-    const bool mci = cin - I * dt / cpv >= 1e-9f;
-    const bool mco = cout + I * dt / (cpv * (float)kEVR) >= 1e-9f;
-    const float lI = -lo[5] - (mci ? lo[3] * dt / cpv : 0.0f) + (mco ? lo[4] * dt / (cpv * (float)kEVR) : 0.0f);
-    const float lopen = lI * Kc * G.F * den;
-    const float lF = lI * Kc * den * open;
-    const float lmv = lo[1] + lopen * do_dm, lhv = lo[2] + lopen * do_dh;
-    const float lVc = lo[0] + lF * G.dV + lmv * dm_dV + lhv * dh_dV;
-    lx[0] = mV ? lVc : 0.0f;
-    lx[1] = lmv * dm_dm;
-    lx[2] = lhv * dh_dh;
-    lx[3] = (mci ? lo[3] : 0.0f) + lF * G.dci;
-    lx[4] = (mco ? lo[4] : 0.0f) + lF * G.dco;
-    lx[5] = lI * Kc * G.F * open;
+    g.open = mv * mv * mv * hv / cdiv;
+    g.do0 = 3.0f * mv * mv * hv / cdiv;
+    g.do1 = mv * mv * mv / cdiv;
+    const float k16 = (float)((double)20.7f * 1e-12 * (kR * kT) / (kF * kF * (double)55.964f) * 1e12);
+    const float k12 = (float)((double)20.8f * 1e-12 * (kR * kT) / (kF * kF * (double)55.964f) * 1e12);
+    g.Kc = (is12 ? k12 : k16) * area;
+    return g;
 }
-
-__device__ __forceinline__ void vjp_kvdr_f(const float* lo, float* lx, float V, float n0, float cin, float cout,
-                                           float den, float area, double vol, float dt, const float* st) {
-    const float V_half = (st[1] != 0.0f) ? st[1] : -30.0f;
-    const float k = (st[2] > 0.0f) ? st[2] : 6.0f;
+__device__ __forceinline__ GateF kvdr_gates_f(float V, float n0, float area, float dt, float st1, float st2, float st4) {
+    GateF g;
+    g.V = V;
+    const float V_half = (st1 != 0.0f) ? st1 : -30.0f;
+    const float k = (st2 > 0.0f) ? st2 : 6.0f;
     float tau, dtau;
-    if (st[4] > 0.0f) { tau = st[4]; dtau = 0.0f; }
+    if (st4 > 0.0f) { tau = st4; dtau = 0.0f; }
     else {
         const float t0 = 14.6f * expf(-(V - V_half) / 30.1f);
         if (t0 < 0.3f) { tau = 0.3f; dtau = 0.0f; }
@@ -704,42 +710,73 @@ __device__ __forceinline__ void vjp_kvdr_f(const float* lo, float* lx, float V, 
     const float tt = tau + 1e-6f;
     const float nu = n0 + (minf - n0) * dt / tt;
     const bool mn = nu >= 0.0f && nu <= 1.0f;
-    const float nv = mn ? nu : (nu < 0.0f ? 0.0f : 1.0f);
-    const float dn_dV = mn ? (dminf * dt / tt - (minf - n0) * dt * dtau / (tt * tt)) : 0.0f;
-    const float dn_dn = mn ? 1.0f - dt / tt : 0.0f;
-    const float Kc = (float)(12.0 * 1e-12 * (kR * kT) / (kF * kF * (double)40.514f) * 1e12) * area;
-    const GhkF G = ghk_mono_f(V, cin, cout);
-    const float I = Kc * G.F * den * nv;
-    const float cpmv = (float)(kF * vol / 1000.0);
-    const bool mci = cin - I * dt / cpmv >= 1e-9f;
-    const bool mco = cout + I * dt / (cpmv * (float)kEVR) >= 1e-9f;
-    const float lI = -lo[5] - (mci ? lo[3] * dt / cpmv : 0.0f) + (mco ? lo[4] * dt / (cpmv * (float)kEVR) : 0.0f);
-    const float lF = lI * Kc * den * nv;
-    const float lnv = lo[1] + lI * Kc * G.F * den;
-    lx[0] = lo[0] + lF * G.dV + lnv * dn_dV;
-    lx[1] = lnv * dn_dn;
-    lx[2] = 0.0f;
-    lx[3] = (mci ? lo[3] : 0.0f) + lF * G.dci;
-    lx[4] = (mco ? lo[4] : 0.0f) + lF * G.dco;
-    lx[5] = lI * Kc * G.F * nv;
+    g.open = mn ? nu : (nu < 0.0f ? 0.0f : 1.0f);
+    g.d0V = mn ? (dminf * dt / tt - (minf - n0) * dt * dtau / (tt * tt)) : 0.0f;
+    g.d00 = mn ? 1.0f - dt / tt : 0.0f;
+    g.do0 = 1.0f;
+    g.do1 = g.d1V = g.d11 = 0.0f;
+    g.Kc = (float)(12.0 * 1e-12 * (kR * kT) / (kF * kF * (double)40.514f) * 1e12) * area;
+    return g;
+}
+__device__ __forceinline__ GateF k2p_gates_f(float V, float area, float st0, float st1) {
+    GateF g;
+    g.V = V;
+    float k = (float)(100.0 * 1e-12 * (kR * kT) / (kF * kF * (double)40.514f) * 1e12 * (double)0.012f);
+    if (st0 > 0.0f || st1 > 0.0f) {
+        const double gamma = (st0 > 0.0f) ? (double)st0 : 100.0;
+        const double Po = (st1 > 0.0f) ? (double)st1 : (double)0.012f;
+        k = (float)(gamma * 1e-12 * (kR * kT) / (kF * kF * (double)40.514f) * 1e12 * Po);
+    }
+    g.Kc = k * area;
+    g.open = 1.0f;   // Po stands in Kc
+    g.do0 = g.do1 = g.d0V = g.d1V = g.d00 = g.d11 = 0.0f;
+    return g;
 }
 
-__device__ __forceinline__ void vjp_k2p_f(const float* lo, float* lx, float V, float cin, float cout, float den,
-                                          float area, double vol, float dt, const float* st) {
-    const double gamma = (st[0] > 0.0f) ? (double)st[0] : 100.0;
-    const double Po = (st[1] > 0.0f) ? (double)st[1] : (double)0.012f;
-    const float Kc = (float)((double)(float)gamma * 1e-12 * (kR * kT) / (kF * kF * (double)40.514f) * 1e12 * Po) * area;
-    const GhkF G = ghk_mono_f(V, cin, cout);
-    const float I = Kc * G.F * den;
-    const float cpv = (float)(kF * vol / 1000.0);
-    const bool mco = cout + I * dt / (cpv * (float)kEVR) >= 1e-9f;
-    const float lI = -lo[5] - lo[3] * dt / cpv + (mco ? lo[4] * dt / (cpv * (float)kEVR) : 0.0f);
-    const float lF = lI * Kc * den;
-    lx[0] = lo[0] + lF * G.dV;
-    lx[1] = lx[2] = 0.0f;
-    lx[3] = lo[3] + lF * G.dci;
+// The Nav, Kv_DR and K2P items (types 141, 142, 123, 107): lx = lo J.  cpv: charge per mole
+// of the segment's volume; st: the item's parameter words, null where all are the
+// defaults.  The current, its ions' clamps and their products are the three
+// models' one copy: the reverse kernel is bound by instruction fetch (2.8 of the 8.6 cycles
+// a warp takes per instruction, a tick's code running once per tick), so the code's length
+// is its time.  Backward pass of 64 neurons x 64 segments, 16 sets, 160 ticks: 65.2 ms with
+// a product per model in line, 61.9 so.
+__device__ __forceinline__ void vjp_item_f(uint8_t type, const float* lo, float* lx, float V0, float x0, float x1,
+                                           float cin, float cout, float den, float area, float cpv, float dt,
+                                           const float* st) {
+    const bool kv = type == 123, k2p = type == 107;
+    GateF g;
+    float p0 = 0.0f, p1 = 0.0f, p2 = 0.0f;
+    if (st) {
+        p0 = st[kv ? 1 : (k2p ? 0 : 5)];
+        if (kv || k2p) p1 = st[kv ? 2 : 1];
+        if (kv) p2 = st[4];
+    }
+    if (kv) g = kvdr_gates_f(V0, x0, area, dt, p0, p1, p2);
+    else if (k2p) g = k2p_gates_f(V0, area, p0, p1);
+    else g = nav_gates_f(V0, x0, x1, area, dt, type == 142 ? 1 : 0, p0);
+    const GhkF G = ghk_mono_f(g.V, cin, cout);
+    const float KF = g.Kc * G.F;
+    const float I = KF * den * g.open;
+    const float cpo = cpv * (float)kEVR;
+    const bool mci = k2p || cin - I * dt / cpv >= 1e-9f;
+    const bool mco = cout + I * dt / cpo >= 1e-9f;
+    const float lI = -lo[5] - (mci ? lo[3] * dt / cpv : 0.0f) + (mco ? lo[4] * dt / cpo : 0.0f);
+    const float lIK = lI * g.Kc;
+    const float lIF = lIK * G.F, lF = lIK * den * g.open;
+    const float lopen = lIF * den;
+    const float l0 = lo[1] + lopen * g.do0, l1 = lo[2] + lopen * g.do1;
+    float lV = lo[0] + lF * G.dV;
+    if (!k2p) lV += l0 * g.d0V;
+    if (!k2p && !kv) {
+        lV += l1 * g.d1V;
+        if (!(V0 >= -200.0f && V0 <= 200.0f)) lV = 0.0f;
+    }
+    lx[0] = lV;
+    lx[1] = l0 * g.d00;
+    lx[2] = l1 * g.d11;
+    lx[3] = (mci ? lo[3] : 0.0f) + lF * G.dci;
     lx[4] = (mco ? lo[4] : 0.0f) + lF * G.dco;
-    lx[5] = lI * Kc * G.F;
+    lx[5] = lIF * g.open;
 }
 
 // Scharfetter-Gummel Bernoulli function B(x) = x / (e^x - 1) and B'(x) in single
