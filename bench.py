@@ -537,7 +537,7 @@ def run_trees(a, device):
                             "ms_per_tick": ms_fixed / a.tree_ticks,
                             "note": "the reference's fixed 50 sweeps per solve (parity mode)"},
         "kernels_ms": {"k_modifiers": ms_mod / n_prof, "k_diffusion": ms_diff / n_prof, "k_synapse": ms_syn / n_prof},
-        "cluster": "2 CTAs per tree (distributed shared memory)", "setup_s": round(setup_s, 1),
+        "cluster": "one CTA per tree", "setup_s": round(setup_s, 1),
         "cpu_reference": cpu,
     }
 
