@@ -149,25 +149,35 @@ struct Lay {
     unsigned long long* pmask;   // reverse pass: per segment, the phi_e sweeps that did not clamp
     float *st, *gax, *term, *vnA, *vnB;
     float* coef;        // [7][Emax] D area dt_sub / length, fixed for the run
-    int* nphi;          // sweeps the phi_e solve ran before its iterate stopped changing
+    int* nphi;          // reverse pass: sweeps the phi_e solve ran before its iterate stopped changing
     uint32_t* itw;      // [items][S] an item's type | its first gate word << 8 | default parameters << 16
     float* iden;        // [items][S] its density
     uint32_t* evc;      // [Y] each synapse's first release at or after the last tick run
+    // coef, itw, iden and evc are in the CTA's scratch in global memory (lean layout) where
+    // a neuron has so many synapses that shared memory would not hold them too
     // reverse pass only
     float *s2, *lam, *lphi, *lI, *mu, *lvB, *linp, *lgdg, *eca, *ecb, *edv, *ldiag, *jsm;
 };
 
-__host__ __device__ inline size_t lay_bytes(uint32_t S, uint32_t E, uint32_t Y, bool bwd, uint32_t W) {
+// Words of the arrays the lean layout keeps in global memory.
+__host__ __device__ inline size_t lean_floats(uint32_t S, uint32_t E, uint32_t Y) {
+    return 7 * (size_t)E + 2 * kItems * (size_t)S + Y;
+}
+
+__host__ __device__ inline size_t lay_bytes(uint32_t S, uint32_t E, uint32_t Y, bool bwd, uint32_t W, bool lean) {
     size_t dbl = (size_t)6 * S + 15 * (size_t)E;
-    size_t flt = (size_t)W * S + kSynWords * Y + 2 * (size_t)E + 2 * (size_t)S + 7 * (size_t)E + 1 + 2 * kItems * (size_t)S + Y;
+    size_t flt = (size_t)W * S + kSynWords * Y + 2 * (size_t)E + 2 * (size_t)S + (lean ? 0u : lean_floats(S, E, Y));
     if (bwd) {
         dbl += S;   // pmask
+        // the last 4: up to 3 to align jsm, and nphi
         flt += 15 * (size_t)S + W * (size_t)S + kSynWords * (size_t)Y + 7 * (size_t)S + (size_t)E + 51 * (size_t)S + 4;
     }
     return dbl * 8 + flt * 4;
 }
 
-__device__ inline Lay make_lay(unsigned char* base, uint32_t S, uint32_t E, uint32_t Y, bool bwd, uint32_t W) {
+// lean: where the arrays of lean_floats go, null for shared memory.
+template <bool kLean>
+__device__ inline Lay make_lay(unsigned char* base, uint32_t S, uint32_t E, uint32_t Y, bool bwd, uint32_t W, float* lean) {
     Lay l;
     double* d = reinterpret_cast<double*>(base);
     l.ibuf = d; d += S; l.phiA = d; d += S; l.phiB = d; d += S; l.sig = d; d += S; l.diag = d; d += S;
@@ -178,11 +188,12 @@ __device__ inline Lay make_lay(unsigned char* base, uint32_t S, uint32_t E, uint
     l.st = f; f += W * S + kSynWords * Y;
     l.gax = f; f += E; l.term = f; f += E;
     l.vnA = f; f += S; l.vnB = f; f += S;
-    l.coef = f; f += 7 * E;
-    l.nphi = reinterpret_cast<int*>(f); f += 1;
-    l.itw = reinterpret_cast<uint32_t*>(f); f += kItems * S;
-    l.iden = f; f += kItems * S;
-    l.evc = reinterpret_cast<uint32_t*>(f); f += Y;
+    float* x = kLean ? lean : f;
+    l.coef = x; x += 7 * E;
+    l.itw = reinterpret_cast<uint32_t*>(x); x += kItems * S;
+    l.iden = x; x += kItems * S;
+    l.evc = reinterpret_cast<uint32_t*>(x); x += Y;
+    if (!kLean) f = x;
     if (bwd) {
         l.s2 = f; f += 15 * S;
         l.lam = f; f += W * S + kSynWords * Y;   // the state's layout: segment words, then synapse words
@@ -194,9 +205,11 @@ __device__ inline Lay make_lay(unsigned char* base, uint32_t S, uint32_t E, uint
         // 16-byte aligned for the asynchronous copies
         f = reinterpret_cast<float*>((reinterpret_cast<uintptr_t>(f) + 15u) & ~(uintptr_t)15u);
         l.jsm = f; f += 51 * S;
+        l.nphi = reinterpret_cast<int*>(f);
     } else {
         l.s2 = l.lam = l.lphi = l.lI = l.mu = l.lvB = l.linp = l.lgdg = l.eca = l.ecb = l.edv = l.ldiag =
             l.jsm = nullptr;
+        l.nphi = nullptr;
     }
     return l;
 }
@@ -487,6 +500,7 @@ struct Scr {
     float* estart;    // [6][7][Sm]  out before each extra sub-step and before the bath
     float* syn;       // [Ymax][kSynScr] in[7] before the synapse, receptor open probabilities, NMDA gates
     float* atpf;      // [Sm]        ATP before the Fick pass
+    float* lean;      // [lean_floats] of the lean layout, at the scratch's end
 };
 // items: the item stride of the kernels; atp: whether the ATP row is recorded
 __host__ __device__ inline size_t scr_floats(uint32_t S, uint32_t Y, uint32_t items, bool atp) {
@@ -506,6 +520,7 @@ __device__ inline Scr make_scr(const AdjDev& d) {
     s.syn = f; f += kSynScr * d.Ymax;
     s.pre = f; f += (size_t)ItemStride<kFull>::v * 5 * S;
     s.atpf = f;
+    s.lean = base + d.scr_floats - lean_floats(S, d.Emax, d.Ymax);
     return s;
 }
 
@@ -1417,7 +1432,7 @@ template <bool kFull, int kThreads, int kMinBlocks>
 __global__ void __launch_bounds__(kThreads, kMinBlocks) k_adj_forward(AdjDev d, uint32_t t0, uint32_t t1) {
     extern __shared__ __align__(16) unsigned char smem[];
     const Ctx c = make_ctx(d);
-    const Lay L = make_lay(smem, d.Smax, d.Emax, d.Ymax, false, d.W);
+    const Lay L = make_lay<false>(smem, d.Smax, d.Emax, d.Ymax, false, d.W, nullptr);
     const Scr sc{};
     float* gstate = d.state + (size_t)c.p * d.L + c.st_off;
     coef_fill(d, c, L);
@@ -1455,7 +1470,7 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) k_adj_rerun(AdjDev d, ui
     extern __shared__ __align__(16) unsigned char smem[];
     const Ctx c = make_ctx(d);
     const uint32_t W = kFull ? d.W : kW3;
-    const Lay L = make_lay(smem, d.Smax, d.Emax, d.Ymax, false, W);
+    const Lay L = make_lay<false>(smem, d.Smax, d.Emax, d.Ymax, false, W, nullptr);
     const Scr sc{};
     const uint32_t tb = w * d.K;
     const uint32_t te = min(d.T, tb + d.K);
@@ -1474,14 +1489,16 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) k_adj_rerun(AdjDev d, ui
 // Reverse pass over window w (ticks [w K, min((w + 1) K, T))), after k_adj_rerun has
 // left each tick's starting state in the window buffer.
 // kThreads / kMinBlocks: the launch bounds (neurons of at most 64 segments run a
-// 64-thread instantiation bounded for 5 CTAs per SM).
-template <bool kFull, int kThreads, int kMinBlocks>
+// 64-thread instantiation bounded for BNC_ADJ_MIN_BLOCKS CTAs per SM).  kLean: the lean
+// layout, for neurons with so many synapses that only one CTA fits an SM anyway (whole
+// small set: 3,180 to 3,714 synapses onto 128 segments, 4,234 to 4,764 onto 64).
+template <bool kFull, int kThreads, int kMinBlocks, bool kLean>
 __global__ void __launch_bounds__(kThreads, kMinBlocks) k_adj_backward(AdjDev d, uint32_t w) {
     extern __shared__ __align__(16) unsigned char smem[];
     const Ctx c = make_ctx(d);
     const uint32_t W = kFull ? d.W : kW3;
-    const Lay L = make_lay(smem, d.Smax, d.Emax, d.Ymax, true, W);
     const Scr sc = make_scr<kFull>(d);
+    const Lay L = make_lay<kLean>(smem, d.Smax, d.Emax, d.Ymax, true, W, sc.lean);
     const uint32_t tb = w * d.K;
     const uint32_t te = min(d.T, tb + d.K);
     const uint32_t Sm = d.Smax;
@@ -1550,6 +1567,7 @@ struct Adjoint {
     AdjDev d{};
     uint32_t threads = 32;
     size_t smem_fwd = 0, smem_bwd = 0;
+    bool lean = false;   // the reverse pass's layout
     // host copies
     std::vector<uint32_t> slot_of_syn;    // original synapse -> slot (UINT32_MAX: not modelled)
     std::vector<uint32_t> soma;           // per neuron: global soma segment
@@ -1928,7 +1946,14 @@ int adj_build(Adjoint* A, void* sim, const BncAdjointConfig& cfg) {
     d.loss_part = static_cast<double*>(al.alloc((size_t)cfg.n_sets * nn * sizeof(double)));
     d.g_par = static_cast<double*>(al.alloc((size_t)cfg.n_sets * 3 * N * sizeof(double)));
     d.g_w = static_cast<double*>(al.alloc((size_t)cfg.n_sets * std::max(KS, 1u) * sizeof(double)));
-    d.scr_floats = scr_floats(d.Smax, Ymax, full_items ? (uint32_t)kItems : 3u, has_atp);
+    constexpr size_t kMaxSmem = 227u * 1024u;
+    A->smem_fwd = lay_bytes(d.Smax, d.Emax, Ymax, false, Wseg, false);   // less than the lean reverse pass's for any neuron
+    A->smem_bwd = lay_bytes(d.Smax, d.Emax, Ymax, true, Wseg, false);
+    A->lean = A->smem_bwd > kMaxSmem;
+    if (A->lean) A->smem_bwd = lay_bytes(d.Smax, d.Emax, Ymax, true, Wseg, true);
+    if (A->smem_bwd > kMaxSmem) { set_error("adjoint: a neuron needs %zu bytes of shared memory", A->smem_bwd); return BNC_ERR_UNSUPPORTED; }
+    d.scr_floats = scr_floats(d.Smax, Ymax, full_items ? (uint32_t)kItems : 3u, has_atp) +
+                   (A->lean ? (lean_floats(d.Smax, d.Emax, Ymax) + 3) & ~(size_t)3 : 0u);
     d.scr = static_cast<float*>(al.alloc((size_t)nn * cfg.n_sets * d.scr_floats * sizeof(float)));
     if (!d.state || !d.lam || !d.ckpt || !d.win || !d.loss_part || !d.g_par || !d.g_w || !d.scr)
         return adj_fail(BNC_ERR_ALLOC, "state, checkpoints and scratch");
@@ -1944,19 +1969,18 @@ int adj_build(Adjoint* A, void* sim, const BncAdjointConfig& cfg) {
     d.target = nullptr;
     d.trace = nullptr;
     A->threads = ((std::max(d.Smax, d.Emax) + 31u) / 32u) * 32u;
-    A->smem_fwd = lay_bytes(d.Smax, d.Emax, Ymax, false, Wseg);
-    A->smem_bwd = lay_bytes(d.Smax, d.Emax, Ymax, true, Wseg);
-    if (A->smem_bwd > 227u * 1024u) { set_error("adjoint: a neuron needs %zu bytes of shared memory", A->smem_bwd); return BNC_ERR_UNSUPPORTED; }
     // the limit is a property of the kernel, not of this object: the most any neuron needs
     const void* kernels[] = {
         (const void*)k_adj_forward<false, kMaxSeg, 1>, (const void*)k_adj_forward<true, kMaxSeg, 1>,
         (const void*)k_adj_forward<false, 64, BNC_ADJ_FWD_BLOCKS>, (const void*)k_adj_forward<true, 64, BNC_ADJ_FWD_BLOCKS>,
         (const void*)k_adj_rerun<false, kMaxSeg, 1>, (const void*)k_adj_rerun<true, kMaxSeg, 1>,
         (const void*)k_adj_rerun<false, 64, BNC_ADJ_FWD_BLOCKS>, (const void*)k_adj_rerun<true, 64, BNC_ADJ_FWD_BLOCKS>,
-        (const void*)k_adj_backward<false, kMaxSeg, 1>, (const void*)k_adj_backward<true, kMaxSeg, 1>,
-        (const void*)k_adj_backward<false, 64, BNC_ADJ_MIN_BLOCKS>, (const void*)k_adj_backward<true, 64, BNC_ADJ_MIN_BLOCKS>};
+        (const void*)k_adj_backward<false, kMaxSeg, 1, false>, (const void*)k_adj_backward<true, kMaxSeg, 1, false>,
+        (const void*)k_adj_backward<false, kMaxSeg, 1, true>, (const void*)k_adj_backward<true, kMaxSeg, 1, true>,
+        (const void*)k_adj_backward<false, 64, BNC_ADJ_MIN_BLOCKS, false>,
+        (const void*)k_adj_backward<true, 64, BNC_ADJ_MIN_BLOCKS, false>};
     for (const void* k : kernels)
-        if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024) != cudaSuccess)
+        if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxSmem) != cudaSuccess)
             return adj_fail(BNC_ERR_CUDA, "shared-memory limit");
     return BNC_OK;
 }
@@ -2192,12 +2216,15 @@ int bnc_adjoint_backward(void* adj, float* g_gNa, float* g_gK, float* g_gleak, f
             if (d.full) k_adj_rerun<true, kMaxSeg, 1><<<grid, A->threads, A->smem_fwd, A->stream>>>(d, (uint32_t)w);
             else k_adj_rerun<false, kMaxSeg, 1><<<grid, A->threads, A->smem_fwd, A->stream>>>(d, (uint32_t)w);
         }
-        if (A->threads <= 64) {
-            if (d.full) k_adj_backward<true, 64, BNC_ADJ_MIN_BLOCKS><<<grid, A->threads, A->smem_bwd, A->stream>>>(d, (uint32_t)w);
-            else k_adj_backward<false, 64, BNC_ADJ_MIN_BLOCKS><<<grid, A->threads, A->smem_bwd, A->stream>>>(d, (uint32_t)w);
+        if (A->lean) {
+            if (d.full) k_adj_backward<true, kMaxSeg, 1, true><<<grid, A->threads, A->smem_bwd, A->stream>>>(d, (uint32_t)w);
+            else k_adj_backward<false, kMaxSeg, 1, true><<<grid, A->threads, A->smem_bwd, A->stream>>>(d, (uint32_t)w);
+        } else if (A->threads <= 64) {
+            if (d.full) k_adj_backward<true, 64, BNC_ADJ_MIN_BLOCKS, false><<<grid, A->threads, A->smem_bwd, A->stream>>>(d, (uint32_t)w);
+            else k_adj_backward<false, 64, BNC_ADJ_MIN_BLOCKS, false><<<grid, A->threads, A->smem_bwd, A->stream>>>(d, (uint32_t)w);
         } else {
-            if (d.full) k_adj_backward<true, kMaxSeg, 1><<<grid, A->threads, A->smem_bwd, A->stream>>>(d, (uint32_t)w);
-            else k_adj_backward<false, kMaxSeg, 1><<<grid, A->threads, A->smem_bwd, A->stream>>>(d, (uint32_t)w);
+            if (d.full) k_adj_backward<true, kMaxSeg, 1, false><<<grid, A->threads, A->smem_bwd, A->stream>>>(d, (uint32_t)w);
+            else k_adj_backward<false, kMaxSeg, 1, false><<<grid, A->threads, A->smem_bwd, A->stream>>>(d, (uint32_t)w);
         }
     }
     cudaEventRecord(A->ev1, A->stream);
