@@ -1122,6 +1122,23 @@ __global__ void k_inject(NetDev d) {
     *d.inj_n = 0u;
 }
 
+// Networks of trees with the options of NetDev::diff_mode that the tile kernel runs faster:
+// components of at most 1,024 segments whose tiles, a thread per segment, are all resident
+// at once.  k_diffusion_tree has half the threads of such a tile, two slots each, which pays
+// when a second wave of tiles would follow, and for one small tile without the ledger.
+// Step 2.5 per tick, tree / tile kernel.  Residual solves: 7 trees of 63 segments 241 / 183
+// us, 1,587 trees 392 / 315, 2,063 (258 tiles of 512 threads) 385 / 310, 2,380 (298) 382 /
+// 387; 117 of 255 331 / 312, 588 (147 tiles of 1,024) 379 / 331, 705 (177) 469 / 587; 146 of
+// 1,023 410 / 343, 175 497 / 563; one of 127 141 / 144, with the ledger 167 / 158.  Ledger
+// alone: 2,000 trees of 15 198 / 177 (63 tiles of 480), 6,666 220 / 226; 476 of 63 194 / 187;
+// 236 of 127 (30 tiles of 1,024) 194 / 239; one of 255 135 / 165.
+static bool options_on_tiles(const NetDev& dev, const NetHost& host) {
+    if (!dev.diff_mode || host.cluster != 1) return false;
+    const uint32_t threads = diffusion_threads(host.max_tile_segs);
+    if (dev.diff_mode & 1u) return (threads > 256u || dev.diff_mode == 3u) && dev.n_tiles <= 148u * (1024u / threads);
+    return threads > 256u && threads <= 512u && dev.n_tiles <= 148u;
+}
+
 cudaError_t enqueue_diffusion(const NetDev& dev, const NetHost& host, float dt, unsigned long long tick,
                               cudaStream_t stream) {
     if (dev.inj) {
@@ -1130,7 +1147,7 @@ cudaError_t enqueue_diffusion(const NetDev& dev, const NetHost& host, float dt, 
         if (e != cudaSuccess) return e;
     }
     if (host.path_slots && dev.diff_mode == 0u) return launch_diffusion_path(dev, host.path_slots, dt, tick, stream);
-    if (host.tree_slots) return launch_diffusion_tree(dev, host.tree_slots, host.tree_inc, dt, tick, stream);
+    if (host.tree_slots && !options_on_tiles(dev, host)) return launch_diffusion_tree(dev, host.tree_slots, host.tree_inc, dt, tick, stream);
     const uint32_t S = host.max_tile_stride, E = host.max_tile_edges;
     const size_t smem = diffusion_smem_bytes(S, E);
     const uint32_t threads = std::max(host.diff_threads, diffusion_threads(host.max_tile_segs));

@@ -13,7 +13,8 @@
 // 1,024 threads and 64 registers).  Step 2.5 per tick, against k_diffusion<2>: 74 trees of
 // 2,047 segments 239 us against 456 (373 with one list of connections unpacked per use,
 // 287 with the rows' addresses folded); 160 trees with the residual-controlled solves and
-// the ledger 1,032 against 2,000.
+// the ledger 1,032 against 2,000.  Smaller trees with these options, few enough for one wave
+// of the tile kernel, run that (options_on_tiles).
 //
 // The arithmetic is k_diffusion's: a connection runs from child to parent (with its ends
 // exchanged, potential differences and fluxes change sign exactly), every sum keeps
