@@ -370,7 +370,7 @@ k_diffusion_tree(NetDev d, float dt, unsigned long long tick) {
                     for (int k = 0; k < kInc; k++) {
                         const uint32_t w = s.w[k];
                         const double fl = (double)t.f[q][w];
-                        const double dq = fast ? over(fl, vf, yv) : fl / vf;
+                        const double dq = fast ? over(fl, vf, yv) : (w == (uint32_t)C ? 0.0 : fl / vf);
                         acc += w == s.x ? -dq : dq;
                     }
                     const float old = t.c[q][s.x];
@@ -562,7 +562,8 @@ k_diffusion_tree(NetDev d, float dt, unsigned long long tick) {
                         for (int k = 0; k < kInc; k++) {
                             const uint32_t w = sl[r].w[k];
                             const double fl = fr[j][w];
-                            const double dq = fast ? 4.0 * over(fl, (double)sl[r].vf, yv[r]) : fl / (double)vx;
+                            const double dq = fast ? 4.0 * over(fl, (double)sl[r].vf, yv[r])
+                                                   : (w == (uint32_t)C ? 0.0 : fl / (double)vx);
                             acc += w == sl[r].x ? -dq : dq;
                         }
                         const float old = t.c[q][sl[r].x];
