@@ -25,8 +25,8 @@
 //    unchanged in every bit, the remaining sweeps of the 50 would too and are not run;
 //  * (float)(0.5 (double)a + ...) of two floats, and a float plus a float rounded through
 //    double, are the float operations (the double keeps 2 x 24 + 2 bits);
-//  * ion 5 has diffusion coefficient 0: its fluxes are zeros unless an operand is not
-//    finite;
+//  * ion 5 has diffusion coefficient 0: its fluxes are zeros unless a concentration or its
+//    product with a Bernoulli value is not finite;
 //  * divisions by a value used many times are Markstein's correction of a * (1 / b)
 //    (div_rn_f), their range conditions checked once per solve or sub-step instead of
 //    per division.  Warps with a value outside them take the kSafe code, which divides.
@@ -466,7 +466,7 @@ k_diffusion_path(NetDev d, float dt, unsigned long long tick) {
                 for (int s = 0; s < R; s++) {
                     const float gv = 3.612f * sigma[s] * ear[s] / edi[s];
                     gax[s] = has[s] ? gv : 0.0f;
-                    ok &= !has[s] || fabsf(dve[s]) < 1e20f;
+                    ok &= !has[s] || fabsf(dve[s]) < 1e18f;   // x times a concentration below 1e20 stays finite
                 }
                 ok = __all_sync(full, ok);
                 __syncwarp();   // the neighbours' fluxes

@@ -332,7 +332,7 @@ k_diffusion_tree(NetDev d, float dt, unsigned long long tick) {
                 }
                 t.gax[s.x] = div_rn_f(3.612f * sigma * area, dist, rdist);
                 t.term[s.x] = dve;   // for now
-                ok &= lo >= 2u * 0x12800000u - 1u && hi <= 0x1p90f && fabsf(dve) < 1e20f;   // 0x12800000: 2^-90
+                ok &= lo >= 2u * 0x12800000u - 1u && hi <= 0x1p90f && fabsf(dve) < 1e18f;   // 0x12800000: 2^-90
             }
         }
         const bool fast = __syncthreads_and(ok) != 0;

@@ -1,6 +1,8 @@
 """Step 2.5 at the edges of what the path and tree kernels' shortened arithmetic covers,
 against the oracle: an isolated segment of NaN size in a network of trees (a missing
-connection adds nothing, whatever the volume).  All tests are marked gpu."""
+connection adds nothing, whatever the volume), and potentials and HCO3- concentrations so
+large that the ion's flux, whose diffusion coefficient is 0, is 0 x infinity.  All tests
+are marked gpu."""
 import numpy as np
 import pytest
 
@@ -43,3 +45,18 @@ def test_isolated_segment_of_no_size(children, radius):
         net.segments["radius"][4 * segs + 7] = radius
         net.segments["modifier_count"][4 * segs + 7] = 0
     _check(segs, change, (1, 3))
+
+
+@pytest.mark.parametrize("children", [1, 2])
+def test_flux_of_an_ion_that_does_not_diffuse(children):
+    segs = 30
+
+    def change(net):
+        _rewire(children, segs)(net)
+        s = net.segments
+        s["modifier_count"][segs:2 * segs] = 0   # nothing clamps the potential
+        s["V_m"][segs + 4] = 9.9e19
+        s["intra_ions"][segs:2 * segs, :7] = 0.0   # no other ion's flux overflows first
+        s["intra_ions"][segs:2 * segs, 5] = 9.9e19
+    ora = _check(segs, change, (1, 1))
+    assert np.isnan(ora.segment_field("ion_in", 5)[segs:2 * segs]).any()
