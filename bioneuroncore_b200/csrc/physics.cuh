@@ -18,7 +18,10 @@ namespace bnc {
 // IBM J. Res. Dev. 34(1)): 27 cycles of latency against 112 for the division, and a third
 // of its instructions.  A NaN the correction makes of an infinite or zero-divided a * y is
 // put back.  Quotients under 2^-900, where the remainder would underflow, may be an ulp
-// off; every use adds the quotient to a float value, which that does not reach.
+// off, and -0 over a positive divisor is +0.  Neither reaches a result: most quotients are
+// added to a value held in float; a GHK flux is zero or above 2^-270 (its numerator is a
+// difference of floats, one of them times at most e^20); phi_e, where the adjoint's replay
+// solves for it, is added to V_m and rounded to float.
 __device__ __forceinline__ double dp_div_y(double a, double b, double y) {
     const double q0 = a * y;
     const double q = __fma_rn(__fma_rn(-q0, b, a), y, q0);
@@ -27,8 +30,8 @@ __device__ __forceinline__ double dp_div_y(double a, double b, double y) {
 // a / c for a constant c: its reciprocal is folded at compile time.
 __device__ __forceinline__ double dp_over(double a, double c) { return dp_div_y(a, c, 1.0 / c); }
 
-// The same in binary32, for dividends that are zero or far from subnormal (a potential less
-// a constant).
+// The same in binary32, for dividends that are zero or above 2^-100 (a potential less a
+// constant, or its square: multiples of 2^-40); each use takes the quotient's exponential.
 __device__ __forceinline__ float fp_over(float a, float c) {
     const float y = 1.0f / c;
     const float q0 = a * y;
