@@ -250,22 +250,6 @@ __device__ __forceinline__ float dp_bz_act(float V, float vh, float k) { return 
 __device__ __forceinline__ float dp_bz_inact(float V, float vh, float k) { return 1.0f / (1.0f + dm_exp(fp_over(V - vh, k))); }
 
 /* ---- gating helpers (modifier_helpers.h:145-215, 264-271, 468-472, 689-702, 1008-1018, 882-892, 909-913, 954-967, 1137-1170, 1188-1210) ---- */
-__device__ __forceinline__ float nav16_am(float V) { return 0.182f * dp_vtrap(V + 43.0f, 6.0f); }
-__device__ __forceinline__ float nav16_bm(float V) { return 0.124f * dp_vtrap(-(V + 43.0f), 6.0f); }
-__device__ __forceinline__ float nav16_ah(float V) { return 0.024f * dp_vtrap(V + 50.0f, 5.0f); }
-__device__ __forceinline__ float nav16_bh(float V) { return 0.0091f * dp_vtrap(-(V + 75.0f), 5.0f); }
-__device__ __forceinline__ float nav16_m_inf(float V) { float a = nav16_am(V), b = nav16_bm(V); return a / (a + b); }
-__device__ __forceinline__ float nav16_m_tau(float V) { return 1.0f / (nav16_am(V) + nav16_bm(V)); }
-__device__ __forceinline__ float nav16_h_inf(float V) { return 1.0f / (1.0f + dm_exp(fp_over(V + 72.0f, 6.2f))); }
-__device__ __forceinline__ float nav16_h_tau(float V) { return 1.0f / (nav16_ah(V) + nav16_bh(V)); }
-__device__ __forceinline__ float nav12_am(float V) { return 0.182f * dp_vtrap(V + 23.0f, 6.0f); }
-__device__ __forceinline__ float nav12_bm(float V) { return 0.124f * dp_vtrap(-(V + 23.0f), 6.0f); }
-__device__ __forceinline__ float nav12_ah(float V) { return 0.024f * dp_vtrap(V + 41.5f, 5.0f); }
-__device__ __forceinline__ float nav12_bh(float V) { return 0.0091f * dp_vtrap(-(V + 66.5f), 5.0f); }
-__device__ __forceinline__ float nav12_m_inf(float V) { float a = nav12_am(V), b = nav12_bm(V); return a / (a + b); }
-__device__ __forceinline__ float nav12_m_tau(float V) { return 1.0f / (nav12_am(V) + nav12_bm(V)); }
-__device__ __forceinline__ float nav12_h_inf(float V) { return 1.0f / (1.0f + dm_exp(fp_over(V + 63.5f, 6.2f))); }
-__device__ __forceinline__ float nav12_h_tau(float V) { return 1.0f / (nav12_ah(V) + nav12_bh(V)); }
 __device__ __forceinline__ float cav21_m_inf(float V) { return 1.0f / (1.0f + dm_exp(fp_over(-(V - -15.0f), 6.0f + 1e-6f))); }
 __device__ __forceinline__ float cav21_h_inf(float V, float Ca_uM) {
     float h = 1.0f / (1.0f + dm_exp((V - -50.0f) / 8.0f));

@@ -114,7 +114,7 @@ __device__ __forceinline__ double receptor_current(const RecKind& K, DMod& m, DS
 // chain, and its latency bounds the synapse step of any network that does not fill the
 // chip many times over.  With the reciprocals a receptor is about 16 dependent FP64
 // operations (9 cycles each) in place of three full divisions (112 cycles each) among 25,
-// and receptor_step runs all four receptor kinds without divergence.
+// and rec_gates, rec_flux and rec_tail run all four receptor kinds without divergence.
 struct RecSeg {
     double A1, D1, y1, e1, o0, o1, o3;   // monovalent: out Na and K times e1, out Cl
     double A2, D2, y2, o2;               // divalent: out Ca times e2
@@ -258,25 +258,7 @@ __device__ __forceinline__ void rec_tail(const RecSeg& f, float ca, float& w, fl
     w = wn < 0.0f ? 0.0f : (wn > 1.0f ? 1.0f : wn);
     It = It * f.mg * ((double)w * (10.0f / (10.0f + 1.0f)));
 }
-// The three in turn, for a receptor at a time (`on`: this lane has one).
-__device__ __forceinline__ bool receptor_step(const RecSeg& f, const RecK& K, int kind, bool on, float den, float area,
-                                              float& r, float& w, float (&in)[7], float dt, float r_inf, float mod_scale,
-                                              double& I) {
-    float rn, wn = w, open, ca;
-    bool ok = rec_gates(K, kind, r, wn, dt, r_inf, rn, open);
-    ok = rec_flux<true>(f, K, kind, ok & f.ok & on, den, area, open, in, dt, mod_scale, I, ca);
-    if (__any_sync(0xFFFFFFFFu, ok & (kind == 1))) {
-        if (kind == 1) rec_tail(f, ca, wn, dt, I);
-    }
-    I = -I;
-    if (ok) {
-        r = rn;
-        w = wn;
-    }
-    return ok;
-}
-
-// receptor_current out of line, for the receptors receptor_step does not hold for.
+// receptor_current out of line, for the receptors the fast form does not hold for.
 struct RecSlow {
     DMod m;
     DSeg s;
