@@ -35,16 +35,35 @@ namespace bnc {
 DeviceAllocs::~DeviceAllocs() { release(); }
 
 void* DeviceAllocs::alloc(size_t bytes) {
-    void* p = nullptr;
-    if (bytes == 0) bytes = 16;
-    if (cudaMalloc(&p, bytes) != cudaSuccess) return nullptr;
-    ptrs.push_back(p);
+    constexpr size_t kAlign = 256, kMinSlab = (size_t)64 << 10, kMaxSlab = (size_t)32 << 20;
+    bytes = (std::max<size_t>(bytes, 16) + kAlign - 1) / kAlign * kAlign;
+    if ((size_t)(end - next) < bytes) {
+        const size_t slab = std::min(std::max(held, kMinSlab), kMaxSlab);
+        const bool own = bytes >= slab / 4;   // an allocation of its own; the slab in use stays
+        void* p = nullptr;
+        size_t size = own ? bytes : slab;
+        if (cudaMalloc(&p, size) != cudaSuccess) {
+            if (own) return nullptr;
+            cudaGetLastError();
+            size = bytes;   // no memory for a slab
+            if (cudaMalloc(&p, size) != cudaSuccess) return nullptr;
+        }
+        ptrs.push_back(p);
+        held += size;
+        if (size == bytes) return p;
+        next = static_cast<unsigned char*>(p);
+        end = next + size;
+    }
+    void* p = next;
+    next += bytes;
     return p;
 }
 
 void DeviceAllocs::release() {
     for (void* p : ptrs) cudaFree(p);
     ptrs.clear();
+    held = 0;
+    next = end = nullptr;
 }
 
 namespace {

@@ -356,8 +356,15 @@ struct Stimuli {
 
 // Builds host-side SoA from AoS and uploads it.  Returns 0 or BNC_ERR_*; on error
 // bnc_last_error() explains.  `dev` receives device pointers (owned by `allocs`).
+// Its arrays share slabs (256-byte aligned, all given back by release): a cudaMalloc of more
+// than about a megabyte takes 0.31 ms and its cudaFree 0.27, whatever the size, and a network
+// has some hundred arrays.  A slab is as large as what is already held, from 64 KB to
+// 32 MB, so that small networks stay with the cheap sizes (17 us) and none holds much over
+// twice what it needs.
 struct DeviceAllocs {
     std::vector<void*> ptrs;
+    size_t held = 0;                            // bytes of ptrs
+    unsigned char *next = nullptr, *end = nullptr;   // what is left of the last slab
     ~DeviceAllocs();
     void* alloc(size_t bytes);
     void release();
