@@ -35,24 +35,22 @@ namespace bnc {
 DeviceAllocs::~DeviceAllocs() { release(); }
 
 void* DeviceAllocs::alloc(size_t bytes) {
-    constexpr size_t kAlign = 256, kMinSlab = (size_t)64 << 10, kMaxSlab = (size_t)32 << 20;
+    constexpr size_t kAlign = 256, kSlabsFrom = (size_t)8 << 20, kMaxSlab = (size_t)32 << 20;
     bytes = (std::max<size_t>(bytes, 16) + kAlign - 1) / kAlign * kAlign;
     if ((size_t)(end - next) < bytes) {
-        const size_t slab = std::min(std::max(held, kMinSlab), kMaxSlab);
-        const bool own = bytes >= slab / 4;   // an allocation of its own; the slab in use stays
+        const size_t slab = std::min(held, kMaxSlab);
+        bool share = held >= kSlabsFrom && bytes < slab / 4;
         void* p = nullptr;
-        size_t size = own ? bytes : slab;
-        if (cudaMalloc(&p, size) != cudaSuccess) {
-            if (own) return nullptr;
-            cudaGetLastError();
-            size = bytes;   // no memory for a slab
-            if (cudaMalloc(&p, size) != cudaSuccess) return nullptr;
+        if (share && cudaMalloc(&p, slab) != cudaSuccess) {
+            cudaGetLastError();   // no memory for a slab
+            share = false;
         }
+        if (!share && cudaMalloc(&p, bytes) != cudaSuccess) return nullptr;
         ptrs.push_back(p);
-        held += size;
-        if (size == bytes) return p;
+        held += share ? slab : bytes;
+        if (!share) return p;   // an allocation of its own; the slab in use stays
         next = static_cast<unsigned char*>(p);
-        end = next + size;
+        end = next + slab;
     }
     void* p = next;
     next += bytes;

@@ -356,11 +356,12 @@ struct Stimuli {
 
 // Builds host-side SoA from AoS and uploads it.  Returns 0 or BNC_ERR_*; on error
 // bnc_last_error() explains.  `dev` receives device pointers (owned by `allocs`).
-// Its arrays share slabs (256-byte aligned, all given back by release): a cudaMalloc of more
-// than about a megabyte takes 0.31 ms and its cudaFree 0.27, whatever the size, and a network
-// has some hundred arrays.  A slab is as large as what is already held, from 64 KB to
-// 32 MB, so that small networks stay with the cheap sizes (17 us) and none holds much over
-// twice what it needs.
+// From 8 MB on its arrays share slabs (256-byte aligned, all given back by release): a
+// cudaMalloc of more than about a megabyte takes 0.31 ms and its cudaFree 0.27, whatever the
+// size, and a network has some hundred arrays.  A slab is as large as what is already held,
+// up to 32 MB, so that no network holds much over twice what it needs.  Below, each array
+// is its own: small ones (17 us) share the driver's 2 MB blocks, and fill those of other
+// networks (2,048 segments beside another such network: 1.8 ms a load, 2.2 with slabs).
 struct DeviceAllocs {
     std::vector<void*> ptrs;
     size_t held = 0;                            // bytes of ptrs
