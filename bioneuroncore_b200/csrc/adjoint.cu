@@ -30,9 +30,9 @@
 //   conductances, the transposed Jacobi sweeps) -> the phi_e solve -> step 1 (local
 //   Jacobians of the channel models by dual numbers, slot order reversed).
 //
-// What bounds it: instruction issue behind latency (forward 43% of issue slots at 14 warps
-// per SM, backward 30% at 8, its 230 registers the limit).  64 neurons x 64 segments, 16
-// sets, 160 ticks: forward 42.2 -> 11.0 ms, backward 139.7 -> 63.2, by what the plain tick
+// What bounds it: latency and instruction fetch (forward 37% of issue slots at 13 warps per
+// SM, backward 25% at 8, its 250 registers the limit).  64 neurons x 64 segments, 16 sets,
+// 160 ticks: forward 42.2 -> 10.9 ms, backward 139.7 -> 60.6, by what the plain tick
 // does too (one Bernoulli pair per valence, corrected quotients, a phi_e solve left at its
 // fixed point), the channel models in line, their items and each synapse's place in the
 // release log in shared memory, two-entry sweeps, and twice the forward CTAs per SM.
@@ -41,8 +41,8 @@
 #define BNC_ADJ_MIN_BLOCKS 4   // CTAs per SM the 64-thread backward is bounded for (5 spills: slower)
 #endif
 #ifndef BNC_ADJ_FWD_BLOCKS
-#define BNC_ADJ_FWD_BLOCKS 8   // and the 64-thread forward and re-run: 128 registers (8: 15.3 ms, 7: 15.1, 10: 18.5,
-#endif                         // 6: 21.1, unbounded at 230 registers: 19.0; 64 neurons x 64, 16 sets, 160 ticks)
+#define BNC_ADJ_FWD_BLOCKS 8   // and the 64-thread forward and re-run: 128 registers (forward at 8: 10.9 ms,
+#endif                         // 7: 10.9, 10: 13.8; backward 60.6, 61.2, 63.3; 64 neurons x 64, 16 sets, 160 ticks)
 #include <algorithm>
 #include <cmath>
 #include <cstring>

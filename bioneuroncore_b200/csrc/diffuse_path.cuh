@@ -6,10 +6,11 @@
 // potentials and the solves' stencils in registers, the ions in the warp's own rows of
 // shared memory, a neighbour's value a register, a shuffle or a row entry away.  No CTA
 // barrier, no incidence lists.  What bounds it is instruction issue and, behind it,
-// instruction fetch (53% of issue slots at 24 warps per SM): about 6,900 instructions per
-// segment and tick, a third of them V_m sweeps at 7 FP32 instructions and 2 / R shuffles,
-// where the CTA-tile kernel runs 27,000 (a sweep there is about 32: shared loads and a
-// store, a barrier, range checks).  So loops over ions and sweeps stay rolled: unrolled,
+// instruction fetch (71% of issue slots at 24 warps per SM and 1.28M segments, 44% in the
+// form for few warps at 55k): about 8,600 lane slots of instructions per segment and tick,
+// a third of them V_m sweeps at 7 FP32 instructions and 2 / R shuffles, where the CTA-tile
+// kernel runs 27,000 (a sweep there is about 32: shared loads and a store, a barrier, range
+// checks).  So loops over ions and sweeps stay rolled: unrolled,
 // 1.28M segments of 64-segment neurons took 502-548 us.
 // Measured, step 2.5 per tick, this kernel against the CTA-tile kernel: 1.28M segments
 // (64 per neuron) 459 us against 1,198; 55k (37 per neuron) 66 against 128; 2,048 (32 per

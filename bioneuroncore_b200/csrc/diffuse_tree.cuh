@@ -9,8 +9,8 @@
 // phi_e and V_m iterates, one ion side at a time (the other waits in the step-1 record or
 // has been written back), the connections' fluxes.
 //
-// What bounds it: instruction issue of the one CTA an SM holds (62% of issue slots at
-// 1,024 threads and 64 registers).  Step 2.5 per tick, against k_diffusion<2>: 74 trees of
+// What bounds it: instruction issue of the one CTA an SM holds (57% of issue slots at
+// 1,024 threads and 64 registers, with and without the options).  Step 2.5 per tick, against k_diffusion<2>: 74 trees of
 // 2,047 segments 239 us against 456 (373 with one list of connections unpacked per use,
 // 287 with the rows' addresses folded); 160 trees with the residual-controlled solves and
 // the ledger 1,032 against 2,000.  Smaller trees with these options, few enough for one wave

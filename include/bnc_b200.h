@@ -301,8 +301,10 @@ int bnc_ensemble_params(uint64_t seed, uint32_t n_members, uint32_t min_segments
 /* Autotuned ensemble load: tries several groupings of components into warp
  * groups and tiles on a strided sample of at most 64 members (build, one untimed
  * tick, then trial_ticks timed with the captured loop), keeps the fastest and
- * builds the whole ensemble with it.  The grouping never changes results.  `out`
- * (may be NULL) receives the choice and its per-tick time on the sample. */
+ * builds the whole ensemble with it.  The grouping never changes results; step 2.5 of
+ * members that are all unbranched paths of at most 128 segments depends on it only
+ * under bnc_set_diffusion_mode, so there the trials differ by noise.
+ * `out` (may be NULL) receives the choice and its per-tick time on the sample. */
 typedef struct {
     uint32_t warp_cap, tile_segs;   /* chosen grouping (segments per warp group / tile) */
     float ms_per_tick;              /* on the sample */

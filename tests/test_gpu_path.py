@@ -1,7 +1,8 @@
 """k_diffusion_path (unbranched networks) against the oracle, bit for bit: component sizes
 at the edges of its lanes and warps, connection lists in any order and direction, and
-values that leave the range of its corrected divisions; beside it the branched networks
-of the same sizes, which keep the CTA-tile kernel.  All tests are marked gpu."""
+values that leave the range of its corrected divisions; beside it networks of the same
+sizes that are not paths: trees (k_diffusion_tree), extracellular connections and cycles
+(the CTA-tile kernel).  All tests are marked gpu."""
 import numpy as np
 import pytest
 
