@@ -120,9 +120,10 @@ def test_chunked_modifier_pass_bitexact(chunk):
 
 @pytest.mark.parametrize("family,cta_barriers", [("small", 0), ("small", 1), ("large", 0), ("large", 1)])
 def test_diffusion_barrier_groups_bitexact(family, cta_barriers):
-    """The diffusion kernel with barriers over a warp (32-segment neurons) or a pair of
-    warps (64-segment neurons), and with CTA-wide barriers: both are the oracle's tick,
-    bit for bit, through releases."""
+    """Unbranched neurons of 32 and of 64 segments by the path kernel (cta_barriers 0, where
+    the tiles planned beside it are grouped by warps or pairs of warps) and by the tile
+    kernel with CTA-wide barriers: both are the oracle's tick, bit for bit, through
+    releases.  test_gpu_tile_forms.py runs the grouped tiles."""
     from bioneuroncore_b200 import Backend, BuildOptions, Network, NetgenParams, NET_LARGE, NET_SMALL
     if family == "small":
         p = NetgenParams(family=NET_SMALL, n_neurons=40, seed=6, flags=32, stim_pA=3000.0)
@@ -174,9 +175,9 @@ def test_fused_modifier_phases_bitexact(fuse):
 
 
 def test_trees_bitexact():
-    """Depth-10 dendritic trees (2,047 segments each) exceed one CTA's tile: each tree
-    runs on a 2-CTA cluster, its halves exchanging ghost segments through distributed
-    shared memory.  The result must still be the oracle's, bit for bit."""
+    """Depth-10 dendritic trees (2,047 segments each), one CTA of the tree kernel each.  They
+    exceed one tile of the tile kernel, whose 2-CTA clusters are planned beside it (n_tiles)
+    and run in test_gpu_tile_forms.py.  The result must be the oracle's, bit for bit."""
     from bioneuroncore_b200 import NetgenParams, NET_TREES
     p = NetgenParams(family=NET_TREES, n_neurons=3, tree_depth=10, seed=8, flags=8)   # perturbed ions
     ora, gpu, net = _pair(p)
@@ -204,7 +205,7 @@ def test_components_split_across_a_cluster_bitexact():
 
 def _mode_net(case):
     from bioneuroncore_b200 import NetgenParams, NET_TREES, NET_LARGE, NET_SMALL, NETGEN_PERTURB_IONS
-    if case == "trees":   # 2,047-segment trees on 2-CTA clusters
+    if case == "trees":   # 2,047-segment trees, a CTA of the tree kernel each
         return NetgenParams(family=NET_TREES, n_neurons=3, tree_depth=10, seed=8, flags=NETGEN_PERTURB_IONS)
     if case == "large":   # one tile holding twelve neurons (twelve convergence groups)
         return NetgenParams(family=NET_LARGE, n_neurons=12, n_synapses=300, seed=5)
